@@ -7,6 +7,7 @@ Translation units are compiled in parallel with nvcc (one -gencode, no cmake):
 * ``bt_step_tma_pal.cu`` — the FP32 fast path with per-voxel rates (rate palette)
 * ``bt_step_f64.cu`` — FP64 step kernels, -fmad=false so that no
   multiply-add contraction changes the reference's rounding
+* ``bt_list.cu``     — builds the pore lists that the list kernels walk
 * ``bt_api.cu``      — host runtime behind include/bt.h
 * ``bt_noalloc.cu``   — the allocation-free single-step entry point
 * ``bt_closure.cu``   — tcgen05 implicit-GEMM 3-D convolution of the learned closure
@@ -39,6 +40,7 @@ UNITS = [
     ("bt_step_tma_pal.cu", ARCH),
     ("bt_step_tma_rf.cu", ARCH + ["--ptxas-options=-v"]),
     ("bt_step_f64.cu", ARCH + ["-fmad=false"]),
+    ("bt_list.cu", ARCH),
     ("bt_api.cu", ARCH),
     ("bt_noalloc.cu", ARCH),
     ("bt_closure.cu", ARCH),

@@ -20,6 +20,7 @@
 
 #include "../../include/bt.h"
 #include "bt_internal.h"
+#include "bt_list.cuh"
 
 namespace {
 
@@ -81,6 +82,10 @@ struct bt_handle {
     // for the next fast step or a finish kernel (on input side fast_side)
     bool fast_pending = false;
     int fast_side = 0;
+    // the same for list steps (they go on across graphs: one closing launch a
+    // run of them)
+    bool list_pending = false;
+    int list_side = 0;
     double* mt_d = nullptr;
     long long mt_cap = 0;
     long long step = 0;
@@ -114,6 +119,21 @@ struct bt_handle {
     std::vector<uint8_t> mask_h;  // host copy of the pore mask (two-component sums)
     uint32_t wait_polls = bt::RING_WAIT_POLLS;  // fast path's plane-ring wait bound
     int phase_axes = bt::PH_ALL;  // KSPACE: axes with a wave vector somewhere in the schedule
+    // the pore list (bt_list.cuh) of the generic kernels, and its chunks
+    bool use_list = false;
+    uint32_t* pidx = nullptr;
+    uint8_t* pcode = nullptr;
+    int* pbox = nullptr;
+    uint32_t npore = 0, pchunks = 1;
+    // The list kernels leave solid voxels alone, which hold zero in both field
+    // buffers unless the caller put something else there: looked over when a
+    // field comes in (solid_flag, pinned: read once the stream is idle) or, after
+    // bt_field_device gave the field away, at the next run. dirty: the buffers
+    // whose solid voxels have to be cleared before a list kernel writes them.
+    int* solid_flag = nullptr;
+    bool solid_unknown = false;
+    bool dirty[2] = {false, false};
+    bool touched = false;         // a field was set, given away or advanced
 };
 
 namespace {
@@ -197,6 +217,9 @@ void fill_params(bt_handle* h, bt::StepParams<T>* p, int zsplit, int zlong = 1 <
             P.an[k] = (T)an[k];
             P.peqn[k] = (T)(c.p_eq * an[k]);
         }
+        P.axis = -1;
+        for (int k = 0; k < 3; ++k)
+            if (an[k] == 1.0 && an[(k + 1) % 3] == 0.0 && an[(k + 2) % 3] == 0.0) P.axis = k;
         P.b = (T)(dTime * c.gamma);
         P.dx = (T)c.dx; P.dy = (T)c.dy; P.dz = (T)c.dz;
         // ExplicitSimple regularises the harmonic mean with 1e-50, the GPU
@@ -240,14 +263,36 @@ void fill_params(bt_handle* h, bt::StepParams<T>* p, int zsplit, int zlong = 1 <
         P.pal_idx = h->pal_ok ? h->pal_idx : nullptr;
         P.wait_polls = h->wait_polls;
         P.phase_axes = h->phase_axes;
+        P.pidx = h->pidx;
+        P.pcode = h->pcode;
+        P.pbox = h->pbox;
+        P.npore = h->npore;
+        P.pchunks = h->pchunks;
+        P.by_pitch = bt::make_fast_div((uint32_t)h->pitch);
+        P.by_ny = bt::make_fast_div((uint32_t)c.ny);
+        P.phw = static_cast<const T*>(h->weights_d);
+        P.part6 = h->part6_d ? h->part6_d + (size_t)s * 6 * h->pchunks : nullptr;
+        P.part6_prev = h->part6_d ? h->part6_d + (size_t)(1 - s) * 6 * h->pchunks : nullptr;
+        P.mt6 = h->mt6_d;
+        P.mt6_cap = h->mt6_cap;
     }
 }
 
 void refresh_params(bt_handle* h) {
+    // list steps keep one partials buffer per input side, as the fast path does
+    const size_t lpart = 3 * (size_t)h->pchunks * h->nb;
     if (h->cfg.precision == BT_F64) {
         fill_params<double>(h, h->pd, h->gzsplit);
+        for (int s = 0; h->use_list && s < 2; ++s) {
+            h->pd[s].partials = h->partials_d + s * lpart;
+            h->pd[s].partials_prev = h->partials_d + (1 - s) * lpart;
+        }
     } else {
         fill_params<float>(h, h->pf, h->gzsplit);
+        for (int s = 0; h->use_list && s < 2; ++s) {
+            h->pf[s].partials = h->partials_d + s * lpart;
+            h->pf[s].partials_prev = h->partials_d + (1 - s) * lpart;
+        }
         fill_params<float>(h, h->pt, h->tzsplit, h->tzlong);
         // the fast path keeps one partials buffer per input side: a step's
         // partials are read by the next step, which writes the other buffer
@@ -333,6 +378,64 @@ long long tma_tiles(const bt_handle* h) {
     return (long long)((c.nx + tw - 1) / tw) * ((c.ny + th - 1) / th);
 }
 
+int grow_partials(bt_handle* h, size_t need) {
+    if (need <= h->partials_cap) return BT_OK;
+    if (h->partials_d) cudaFree(h->partials_d);
+    h->partials_d = nullptr;
+    h->partials_cap = 0;
+    CK(h, cudaMalloc(&h->partials_d, sizeof(double) * need));
+    h->partials_cap = need;
+    return BT_OK;
+}
+
+// the pore list of the generic kernels from the geometry code, in chunks of
+// one or more entries a thread; grids beyond its 31-bit element index (or with
+// edges whose KSPACE phase tables do not fit shared memory) keep the dense
+// kernels
+int build_pore_list(bt_handle* h) {
+    const bt_config& c = h->cfg;
+    h->use_list = false;
+    if (h->pidx) cudaFree(h->pidx);
+    if (h->pcode) cudaFree(h->pcode);
+    if (h->pbox) cudaFree(h->pbox);
+    h->pidx = nullptr;
+    h->pcode = nullptr;
+    h->pbox = nullptr;
+    if (h->comp >= ((size_t)1 << 31)) return BT_OK;
+    if (c.scheme == BT_SCHEME_KSPACE && 2 * h->esz * ((size_t)c.nx + c.ny + c.nz) > 160 * 1024) return BT_OK;
+    const uint32_t nseg = bt::list_segments(c.nx, c.ny, c.nz);
+    uint32_t* offs = nullptr;
+    CK(h, cudaMalloc(&offs, sizeof(uint32_t) * ((size_t)nseg + 1)));
+    cudaError_t e = bt::list_offsets(h->code, c.nx, c.ny, c.nz, h->cpitch, false, offs, h->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h->npore, offs + nseg, 4, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    const size_t n = std::max<size_t>(1, h->npore);
+    if (e == cudaSuccess) e = cudaMalloc(&h->pidx, 4 * n);
+    if (e == cudaSuccess) e = cudaMalloc(&h->pcode, n);
+    if (e == cudaSuccess)
+        e = bt::fill_pore_list(h->code, c.nx, c.ny, c.nz, h->pitch, h->cpitch, offs, h->pidx, h->pcode, h->stream);
+    h->pchunks = (uint32_t)std::min<size_t>((n + bt::LIST_THREADS - 1) / bt::LIST_THREADS,
+                                            (size_t)bt::list_ctas_per_sm(h->esz) * h->num_sms);
+    if (e == cudaSuccess && c.scheme == BT_SCHEME_KSPACE) {
+        e = cudaMalloc(&h->pbox, sizeof(int) * 6 * h->pchunks);
+        if (e == cudaSuccess)
+            e = bt::chunk_boxes(h->pidx, h->npore, h->pchunks, bt::make_fast_div((uint32_t)h->pitch),
+                                bt::make_fast_div((uint32_t)c.ny), h->pitch, c.ny, h->pbox, h->stream);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    cudaFree(offs);
+    CK(h, e);
+    int rc = grow_partials(h, 6 * (size_t)h->pchunks * h->nb);
+    if (rc) return rc;
+    if (h->part6_d) {
+        cudaFree(h->part6_d);
+        h->part6_d = nullptr;
+        CK(h, cudaMalloc(&h->part6_d, sizeof(double) * 6 * std::max<size_t>(SUMS_BLOCKS, 2 * (size_t)h->pchunks)));
+    }
+    h->use_list = true;
+    return BT_OK;
+}
+
 // the fast path's z-chunking: `chunks` chunks per field in total, spread over
 // the tile columns so that they differ by at most one (at least one chunk per
 // column, at most one plane per chunk, chunks of at most 1024 planes)
@@ -352,14 +455,8 @@ int set_tma_chunks(bt_handle* h, long long chunks) {
     h->tzlong = zlong;
     h->tgrid = dim3(zsplit * h->nb, gx, gy);
     h->tpart = 3 * (size_t)zsplit * gx * gy * h->nb;
-    const size_t need = 2 * h->tpart;
-    if (need > h->partials_cap) {
-        if (h->partials_d) cudaFree(h->partials_d);
-        h->partials_d = nullptr;
-        h->partials_cap = 0;
-        CK(h, cudaMalloc(&h->partials_d, sizeof(double) * need));
-        h->partials_cap = need;
-    }
+    int rc = grow_partials(h, 2 * h->tpart);
+    if (rc) return rc;
     refresh_params(h);
     return BT_OK;
 }
@@ -401,6 +498,15 @@ cudaError_t finish_fast(bt_handle* h) {
     return bt::launch_tma_finish(h->pt[h->fast_side], h->tgrid, h->stream);
 }
 
+// close a run of list steps
+cudaError_t finish_list(bt_handle* h) {
+    if (!h->list_pending) return cudaSuccess;
+    h->list_pending = false;
+    h->launches++;
+    return h->cfg.precision == BT_F64 ? bt::launch_list_finish<double>(h->pd[h->list_side], h->stream)
+                                      : bt::launch_list_finish<float>(h->pf[h->list_side], h->stream);
+}
+
 cudaError_t launch_one(bt_handle* h, int side, long long abs_step) {
     const bt_config& c = h->cfg;
     const int prec = (c.scheme != BT_SCHEME_KSPACE && c.vector_mult == 1) ? 1 : 0;
@@ -408,10 +514,27 @@ cudaError_t launch_one(bt_handle* h, int side, long long abs_step) {
     // a pulse step runs on the fast path when all its pulses are fixed-angle
     // (one rotation; not with the rate palette)
     const bool pulse = step_has_pulse(h, abs_step);
+    // (two-component sums are part of the list kernels)
     const bool fast = c.precision == BT_F32 && c.scheme != BT_SCHEME_MACCORMACK && h->use_tma && !h->fields_d &&
+                      !(h->use_list && h->weights_d) &&
                       (!pulse || (!h->pal_ok && h->steps_h[abs_step * h->nb].rot_ok));
     cudaError_t e;
+    if (h->dirty[1 - side]) {
+        // the output buffer holds a field with something in its solid voxels;
+        // the dense kernels write them
+        h->dirty[1 - side] = false;
+        if (!fast && h->use_list) {
+            h->launches++;
+            e = c.precision == BT_F64 ? bt::solid_clear<double>((double*)h->state_base[1 - side], h->code, c.nx, c.ny, c.nz,
+                                                                h->pitch, h->cpitch, (long long)h->comp, h->nb, h->stream)
+                                      : bt::solid_clear<float>((float*)h->state_base[1 - side], h->code, c.nx, c.ny, c.nz,
+                                                               h->pitch, h->cpitch, (long long)h->comp, h->nb, h->stream);
+            if (e != cudaSuccess) return e;
+        }
+    }
     if (fast) {
+        e = finish_list(h);
+        if (e != cudaSuccess) return e;
         // a fast step after a fast step adds its predecessor's partials
         h->launches++;
         e = bt::launch_step_tma(h->pt[side], h->maps[side], c.scheme, vel, prec, h->pal_ok, pulse, h->tgrid,
@@ -429,15 +552,25 @@ cudaError_t launch_one(bt_handle* h, int side, long long abs_step) {
             char* pb = static_cast<char*>(h->pred_base);
             if (c.precision == BT_F64) {
                 double* pr[3] = {(double*)pb, (double*)(pb + 8 * h->comp), (double*)(pb + 16 * h->comp)};
-                e = bt::launch_mac<double>(h->pd[side], pr, vel, prec, h->grid, h->stream);
+                e = h->use_list ? bt::launch_mac_list<double>(h->pd[side], pr, vel, prec, h->stream)
+                                : bt::launch_mac<double>(h->pd[side], pr, vel, prec, h->grid, h->stream);
             } else {
                 float* pr[3] = {(float*)pb, (float*)(pb + 4 * h->comp), (float*)(pb + 8 * h->comp)};
-                e = bt::launch_mac<float>(h->pf[side], pr, vel, prec, h->grid, h->stream);
+                e = h->use_list ? bt::launch_mac_list<float>(h->pf[side], pr, vel, prec, h->stream)
+                                : bt::launch_mac<float>(h->pf[side], pr, vel, prec, h->grid, h->stream);
             }
+        } else if (h->use_list) {
+            e = c.precision == BT_F64 ? bt::launch_step_list<double>(h->pd[side], c.scheme, vel, prec, h->stream)
+                                      : bt::launch_step_list<float>(h->pf[side], c.scheme, vel, prec, h->stream);
         } else if (c.precision == BT_F64)
             e = bt::launch_step<double>(h->pd[side], c.scheme, vel, prec, h->grid, h->stream);
         else
             e = bt::launch_step<float>(h->pf[side], c.scheme, vel, prec, h->grid, h->stream);
+    }
+    if (!fast && h->use_list) {
+        h->list_pending = true;
+        h->list_side = side;
+        return e;
     }
     if (e != cudaSuccess || !h->weights_d) return e;
     // two-component sums of the field this step wrote
@@ -450,6 +583,12 @@ cudaError_t launch_one(bt_handle* h, int side, long long abs_step) {
     const float* w = static_cast<const float*>(h->weights_d);
     return bt::launch_phase_sums<float>(h->pf[side], w, w + h->comp, h->part6_d, SUMS_BLOCKS, h->mt6_d, h->mt6_cap,
                                         h->stream);
+}
+
+// every step of this handle is a list step (no fast path, or nothing for it)
+bool lists_only(const bt_handle* h) {
+    return h->use_list && !(h->cfg.precision == BT_F32 && h->cfg.scheme != BT_SCHEME_MACCORMACK && h->use_tma &&
+                            !h->fields_d && !h->weights_d);
 }
 
 // per-step table: gradient, KSPACE wave vector and face phases, pulse ranges
@@ -583,6 +722,7 @@ int ensure_mt(bt_handle* h, long long n) {
         drop_graphs(h);  // captured launches hold the old buffer
         CK(h, cudaMalloc(&h->mt6_d, sizeof(double) * 6 * cap));
         h->mt6_cap = cap;
+        refresh_params(h);
     }
     if (n <= h->mt_cap) return BT_OK;
     long long cap = std::max<long long>(n, 1024);
@@ -777,6 +917,35 @@ int get_components(bt_handle* h, double* const* dst, const void* const* src, int
     return BT_OK;
 }
 
+// the stream is idle: what the last look at the current field found
+void take_solid_flag(bt_handle* h) {
+    if (*h->solid_flag) h->dirty[h->cur] = true;
+    *h->solid_flag = 0;
+}
+
+// The current field's solid voxels looked over on the device (see solid_flag);
+// with src, the dense device arrays become the field on the way.
+int solid_check(bt_handle* h, const void* const* src) {
+    const bt_config& c = h->cfg;
+    cudaError_t e;
+    if (c.precision == BT_F64) {
+        const double* s[3] = {src ? (const double*)src[0] : nullptr, src ? (const double*)src[1] : nullptr,
+                              src ? (const double*)src[2] : nullptr};
+        e = bt::field_in<double>((double*)h->state_base[h->cur], src ? s : nullptr, h->code, c.nx, c.ny, c.nz, h->pitch,
+                                 h->cpitch, (long long)h->comp, h->nb, h->solid_flag, h->stream);
+    } else {
+        const float* s[3] = {src ? (const float*)src[0] : nullptr, src ? (const float*)src[1] : nullptr,
+                             src ? (const float*)src[2] : nullptr};
+        e = bt::field_in<float>((float*)h->state_base[h->cur], src ? s : nullptr, h->code, c.nx, c.ny, c.nz, h->pitch,
+                                h->cpitch, (long long)h->comp, h->nb, h->solid_flag, h->stream);
+    }
+    CK(h, e);
+    h->launches++;
+    h->touched = true;
+    h->solid_unknown = false;
+    return BT_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -805,7 +974,9 @@ int bt_create(const bt_config* cfg, bt_handle** out) {
     h->pitch = round_up(cfg->nx, 4);
     h->vxpitch = round_up(cfg->nx + 1, 4);
     h->cpitch = round_up(cfg->nx, 16);
-    h->comp = (size_t)h->pitch * cfg->ny * cfg->nz;
+    // elements from one component to the next: 128-byte aligned, with 128 bytes
+    // of zeros behind the last row that no kernel writes
+    h->comp = ((size_t)h->pitch * cfg->ny * cfg->nz + 31) / 32 * 32 + 32;
     h->nb = cfg->batch > 1 ? cfg->batch : 1;
     int rc = BT_OK;
     auto bail = [&](int code) {
@@ -868,6 +1039,8 @@ int bt_create(const bt_config* cfg, bt_handle** out) {
     if (cudaMalloc(&h->ctl_d, sizeof(bt::Ctl)) != cudaSuccess) return bail(BT_E_NOMEM);
     if (cudaMallocHost(&h->ctl_h, sizeof(bt::Ctl)) != cudaSuccess) return bail(BT_E_NOMEM);
     std::memset(h->ctl_h, 0, sizeof(bt::Ctl));
+    if (cudaMallocHost(&h->solid_flag, sizeof(int)) != cudaSuccess) return bail(BT_E_NOMEM);
+    *h->solid_flag = 0;
     if (cudaMemcpy(h->ctl_d, h->ctl_h, sizeof(bt::Ctl), cudaMemcpyHostToDevice) != cudaSuccess) return bail(BT_E_CUDA);
     h->tgrid = dim3(1, 1, 1);
     rc = ensure_mt(h, 1024);
@@ -901,6 +1074,10 @@ int bt_destroy(bt_handle* h) {
     if (h->pulses_d) cudaFree(h->pulses_d);
     if (h->ctl_d) cudaFree(h->ctl_d);
     if (h->ctl_h) cudaFreeHost(h->ctl_h);
+    if (h->solid_flag) cudaFreeHost(h->solid_flag);
+    if (h->pidx) cudaFree(h->pidx);
+    if (h->pcode) cudaFree(h->pcode);
+    if (h->pbox) cudaFree(h->pbox);
     if (h->staging) pinned_put(h->device, h->staging_bytes, h->staging);
     for (auto& e : h->stage_ev)
         if (e) cudaEventDestroy(e);
@@ -968,6 +1145,17 @@ int bt_upload_geometry(bt_handle* h, const uint8_t* mask, const double* vx, cons
             CK(h, cudaStreamSynchronize(h->stream));
         }
     }
+    // a field from before the new geometry may hold something where there is
+    // solid now
+    if (h->touched) {
+        const size_t sbytes = 3 * h->esz * h->comp * h->nb;
+        CK(h, cudaMemsetAsync(h->state_base[1 - h->cur], 0, sbytes, h->stream));
+        if (h->pred_base) CK(h, cudaMemsetAsync(h->pred_base, 0, sbytes, h->stream));
+        h->dirty[1 - h->cur] = false;
+        h->solid_unknown = true;
+    }
+    int rc = build_pore_list(h);
+    if (rc) return rc;
     h->geometry = true;
     if (fast_path_config(h->cfg) && h->tgrid.y > 0) h->use_tma = build_maps(h);
     refresh_params(h);
@@ -1015,6 +1203,8 @@ int bt_set_state(bt_handle* h, const double* mx, const double* my, const double*
                 if (rc) return rc;
             }
     }
+    int rcf = solid_check(h, nullptr);
+    if (rcf) return rcf;
     // FP32: the host arrays have been read (converted into the staging
     // slots); the copies and the frame change complete in the handle's
     // stream order. FP64 copies read the caller's arrays directly, so they
@@ -1030,11 +1220,9 @@ int bt_set_state_device(bt_handle* h, const void* mx, const void* my, const void
     if (!h->geometry) return fail(h, BT_E_STATE, "bt_upload_geometry first");
     const bt_config& c = h->cfg;
     const void* src[3] = {mx, my, mz};
-    for (int b = 0; b < h->nb; ++b)
-        for (int a = 0; a < 3; ++a)
-            CK(h, cudaMemcpy2DAsync((char*)h->state[h->cur][a] + (size_t)b * 3 * h->comp * h->esz, h->pitch * h->esz,
-                                    (const char*)src[a] + (size_t)b * h->nvox * h->esz, c.nx * h->esz, c.nx * h->esz,
-                                    (size_t)c.ny * c.nz, cudaMemcpyDeviceToDevice, h->stream));
+    (void)c;
+    int rc = solid_check(h, src);
+    if (rc) return rc;
     return frame_change(h, h->state[h->cur], +1);
 }
 
@@ -1059,7 +1247,12 @@ int bt_get_state(bt_handle* h, double* mx, double* my, double* mz) {
             to.push_back(dst[a] + (size_t)b * h->nvox);
             fr.push_back((const char*)from[a] + (size_t)b * 3 * h->comp * h->esz);
         }
-    return get_components(h, to.data(), fr.data(), (int)to.size());
+    const int rc = get_components(h, to.data(), fr.data(), (int)to.size());
+    if (rc || !phase) return rc;
+    // the idle buffer now holds the current field's solid voxels too
+    take_solid_flag(h);
+    h->dirty[1 - h->cur] = h->dirty[1 - h->cur] || h->solid_unknown || h->dirty[h->cur];
+    return BT_OK;
 }
 
 int bt_set_schedule(bt_handle* h, const bt_pulse* pulses, int npulses, const double* grad_wave, long long nwave) {
@@ -1093,14 +1286,18 @@ int run_begin(bt_handle* h, long long nsteps) {
         return fail(h, BT_E_ARG, "KSPACE with a gradient needs a waveform covering every step run");
     int rc = ensure_mt(h, nsteps);
     if (rc) return rc;
+    if (h->solid_unknown && (rc = solid_check(h, nullptr))) return rc;
     // ctl: step and mt_base for this run (written in stream order)
     CK(h, cudaStreamSynchronize(h->stream));
+    take_solid_flag(h);
+    h->touched = true;
     h->ctl_h->step = h->step;
     h->ctl_h->mt_base = h->step;
     h->ctl_h->ticket = 0;
     h->ctl_h->status = 0;
+    h->ctl_h->fstep[0] = h->ctl_h->fstep[1] = h->ctl_h->gen_from = h->step;
     CK(h, cudaMemcpyAsync(h->ctl_d, h->ctl_h, sizeof(bt::Ctl), cudaMemcpyHostToDevice, h->stream));
-    h->fast_pending = false;  // a run that failed part-way may have left one
+    h->fast_pending = h->list_pending = false;  // a run that failed part-way may have left one
     h->last_run = nsteps;
     return BT_OK;
 }
@@ -1111,11 +1308,13 @@ int run_begin(bt_handle* h, long long nsteps) {
 int run_advance(bt_handle* h, long long* s, long long end, long long limit) {
     const long long stop = std::min(end, *s + limit);
     while (*s < stop) {
-        bool clean = stop - *s >= GRAPH_STEPS;
+        bool clean = stop - *s >= GRAPH_STEPS && !h->dirty[0] && !h->dirty[1];
         for (long long q = *s; clean && q < *s + GRAPH_STEPS; ++q) clean = !step_has_pulse(h, q);
         if (clean) {
-            // a graph starts and ends with no fast step pending
+            // a graph starts and ends with no fast step pending; list steps go on
             CK(h, finish_fast(h));
+            const bool listed = lists_only(h);
+            if (!listed) CK(h, finish_list(h));
             cudaGraphExec_t& g = h->graph[h->cur];
             if (!g) {
                 cudaGraph_t graph;
@@ -1124,7 +1323,8 @@ int run_advance(bt_handle* h, long long* s, long long end, long long limit) {
                 const long long before = h->launches;
                 for (int q = 0; q < GRAPH_STEPS && e == cudaSuccess; ++q) e = launch_one(h, (h->cur + q) & 1, *s + q);
                 if (e == cudaSuccess) e = finish_fast(h);
-                h->fast_pending = false;
+                if (e == cudaSuccess && !listed) e = finish_list(h);
+                h->fast_pending = h->list_pending = false;
                 h->graph_launches[h->cur] = h->launches - before;
                 h->launches = before;
                 cudaError_t e2 = cudaStreamEndCapture(h->stream, &graph);
@@ -1136,6 +1336,8 @@ int run_advance(bt_handle* h, long long* s, long long end, long long limit) {
             }
             CK(h, cudaGraphLaunch(g, h->stream));
             h->launches += h->graph_launches[h->cur];
+            h->list_pending = listed;
+            h->list_side = 1 - h->cur;  // of the graph's last step
             *s += GRAPH_STEPS;
         } else {
             CK(h, launch_one(h, h->cur, *s));
@@ -1144,6 +1346,7 @@ int run_advance(bt_handle* h, long long* s, long long end, long long limit) {
         }
     }
     CK(h, finish_fast(h));
+    CK(h, finish_list(h));
     h->step = *s;
     return BT_OK;
 }
@@ -1242,10 +1445,12 @@ int bt_measure(bt_handle* h, double* sums3) {
         cudaError_t e;
         if (h->esz == 8) {
             bt::StepParams<double> P = h->pd[h->cur];
+            P.partials = h->partials_d;
             for (int a = 0; a < 3; ++a) P.in[a] += (size_t)b * 3 * h->comp;
             e = bt::launch_sums<double>(P, kv, h->stream);
         } else {
             bt::StepParams<float> P = h->pf[h->cur];
+            P.partials = h->partials_d;
             for (int a = 0; a < 3; ++a) P.in[a] += (size_t)b * 3 * h->comp;
             e = bt::launch_sums<float>(P, kv, h->stream);
         }
@@ -1516,6 +1721,7 @@ int bt_set_phase_weights(bt_handle* h, const double* c1, const double* c2) {
         if (h->part6_d) cudaFree(h->part6_d);
         h->weights_d = nullptr;
         h->part6_d = nullptr;
+        refresh_params(h);
         return BT_OK;
     }
     if (!c1 || !c2) return fail(h, BT_E_ARG, "c1 and c2 are set together");
@@ -1542,7 +1748,8 @@ int bt_set_phase_weights(bt_handle* h, const double* c1, const double* c2) {
         CK(h, cudaStreamSynchronize(h->stream));
         drop_graphs(h);
         CK(h, cudaMalloc(&h->weights_d, 2 * comp * h->esz));
-        CK(h, cudaMalloc(&h->part6_d, sizeof(double) * 6 * SUMS_BLOCKS));
+        CK(h, cudaMalloc(&h->part6_d, sizeof(double) * 6 * std::max<size_t>(SUMS_BLOCKS, 2 * (size_t)h->pchunks)));
+        refresh_params(h);
     }
     return put_pitched(h, h->weights_d, buf, 2);
 }
@@ -1559,6 +1766,8 @@ int bt_read_mt_phases(bt_handle* h, double* out, long long nsteps) {
 int bt_field_device(bt_handle* h, int member, void** mx, void** my, void** mz, int* pitch) {
     if (!h || member < 0 || member >= h->nb || !mx || !my || !mz || !pitch) return fail(h, BT_E_ARG, "bad field query");
     const size_t off = (size_t)member * 3 * h->comp * h->esz;
+    h->solid_unknown = true;  // the caller may write it
+    h->touched = true;
     *mx = (char*)h->state[h->cur][0] + off;
     *my = (char*)h->state[h->cur][1] + off;
     *mz = (char*)h->state[h->cur][2] + off;
@@ -1656,6 +1865,7 @@ int bt_autotune(bt_handle* h, int trial_steps, int* best_chunks) {
     h->cur = cur0;
     cudaMemcpy(h->state_base[h->cur], keep, sbytes, cudaMemcpyDeviceToDevice);
     cudaFree(keep);
+    h->solid_unknown = true;
     if (rc) return rc;
     rc = set_tma_chunks(h, best_ch);
     if (rc) return rc;

@@ -83,6 +83,12 @@ struct DevPulse {
     double eff;       // |axis| (flag 3's effective gradient)
 };
 
+// Division of 31-bit numbers by an invariant (bt_list.cuh, fast_div); mul = 0
+// divides by one.
+struct FastDiv {
+    uint32_t mul, shift;
+};
+
 // Device-side run control: the step index advances inside the kernels so a
 // captured CUDA graph can be replayed for any number of steps.
 struct Ctl {
@@ -95,6 +101,10 @@ struct Ctl {
     // fstep[s] and writes fstep[1 - s]; step is brought up to date by the
     // finish kernel that closes the run)
     long long fstep[2];
+    // list kernels, inside a run of consecutive list steps: the first step whose
+    // sums are not closed yet (each step's are added by the next one, the last
+    // one's by the run's closing launch)
+    long long gen_from;
 };
 
 // Device layouts are pitched so that every row starts on a 16-byte boundary
@@ -120,6 +130,7 @@ struct StepParams {
     // reference's operation order, then rounded to T
     T hx, hy, hz, hxx, hyy, hzz;
     T an[3];                    // unit main-field axis
+    int axis;                   // the axis it lies along exactly (0, 1, 2), else -1
     T peqn[3];                  // pEq * an
     T b;                        // dTime * g
     T dx, dy, dz;
@@ -155,6 +166,22 @@ struct StepParams {
     // FP32 fast path: polls before a plane-ring wait gives up (RING_WAIT_POLLS
     // unless a test shortens it to see the timeout path run)
     uint32_t wait_polls;
+    // list kernels: the pore voxels in list order (element index within a
+    // component, geometry code), each chunk's bounding box [6] (x0, x1, y0, y1,
+    // z0, z1; KSPACE phase tables), divisions by the pitch and by ny
+    const uint32_t* pidx;
+    const uint8_t* pcode;
+    const int* pbox;
+    uint32_t npore;
+    uint32_t pchunks;           // chunks of the list per batch member
+    FastDiv by_pitch, by_ny;
+    // two-component sums (OutputX/Y/Z with NCOMP 2): weights [2][nz][ny][pitch],
+    // block partials, M(t) x 6; null when switched off
+    const T* phw;
+    double* part6;              // this input side's; the previous step's
+    const double* part6_prev;
+    double* mt6;
+    long long mt6_cap;
 };
 
 // TMA descriptors of the FP32 fast path (one per ping-pong input side)
@@ -173,6 +200,15 @@ cudaError_t launch_sums(const StepParams<T>& p, double* out4, cudaStream_t s);
 // MacCormack step (predictor into pred, then corrector into p.out)
 template <typename T>
 cudaError_t launch_mac(const StepParams<T>& p, T* const pred[3], int vel, int prec, dim3 grid, cudaStream_t s);
+// the same steps over the pore list (p.pidx), with the two-component sums when
+// p.phw is set
+template <typename T>
+cudaError_t launch_step_list(const StepParams<T>& p, int scheme, int vel, int prec, cudaStream_t s);
+template <typename T>
+cudaError_t launch_mac_list(const StepParams<T>& p, T* const pred[3], int vel, int prec, cudaStream_t s);
+// closes a run of list steps (p: the last one's parameters): its sums, Ctl::step
+template <typename T>
+cudaError_t launch_list_finish(const StepParams<T>& p, cudaStream_t s);
 // two-component weighted sums of the newest field into mt6 (6 per step)
 template <typename T>
 cudaError_t launch_phase_sums(const StepParams<T>& p, const T* w1, const T* w2, double* part6, int nblocks,

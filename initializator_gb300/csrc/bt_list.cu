@@ -1,0 +1,267 @@
+// Builds the lists of bt_list.cuh on the device from the geometry code.
+#include "bt_list.cuh"
+
+namespace bt {
+
+namespace {
+
+// geometry code of the four voxels of group (xq, y, z); zero outside
+__device__ __forceinline__ uint32_t code4_at(const uint8_t* code, int xq, int y, int z, int nx, int ny, int nz, int cpitch) {
+    if (4 * xq >= nx || xq < 0 || y < 0 || y >= ny || z < 0 || z >= nz) return 0u;
+    return *reinterpret_cast<const uint32_t*>(code + ((long long)z * ny + y) * cpitch + 4 * xq);
+}
+
+constexpr uint32_t PORES = 0x40404040u;
+constexpr int SEG_GROUPS = LT_Q * LT_Y;  // groups of four in one plane of a list column
+static_assert(SEG_GROUPS % 32 == 0, "a warp walks a segment");
+
+struct ListGrid {
+    int nx, ny, nz, pitch, cpitch, ncx;  // ncx: list columns along x
+    uint32_t nseg;                       // segments: column (x fastest) * nz + z
+};
+
+__device__ __forceinline__ void segment_origin(const ListGrid& g, uint32_t s, int& xq0, int& y0, int& z) {
+    z = (int)(s % (uint32_t)g.nz);
+    const uint32_t col = s / (uint32_t)g.nz;
+    xq0 = (int)(col % (uint32_t)g.ncx) * LT_Q;
+    y0 = (int)(col / (uint32_t)g.ncx) * LT_Y;
+}
+
+// one warp a segment: its pore voxels or its groups that hold one
+__global__ void list_count_kernel(const uint8_t* code, ListGrid g, int groups, uint32_t* counts) {
+    const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x & 31;
+    if (s >= g.nseg) return;
+    int xq0, y0, z;
+    segment_origin(g, s, xq0, y0, z);
+    uint32_t n = 0;
+    for (int k = lane; k < SEG_GROUPS; k += 32) {
+        const uint32_t c = code4_at(code, xq0 + k % LT_Q, y0 + k / LT_Q, z, g.nx, g.ny, g.nz, g.cpitch) & PORES;
+        n += groups ? (c ? 1u : 0u) : (uint32_t)__popc(c);
+    }
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0) counts[s] = n;
+}
+
+// one CTA: counts[0..n) -> exclusive sums in place, the total in counts[n]
+__global__ void __launch_bounds__(1024) list_scan_kernel(uint32_t* counts, uint32_t n) {
+    __shared__ uint32_t warp_sum[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t base = 0;
+    for (uint32_t at = 0; at < n; at += 1024 * 4) {
+        uint32_t v[4], t = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t i = at + 4 * tid + k;
+            v[k] = i < n ? counts[i] : 0u;
+            t += v[k];
+        }
+        uint32_t inc = t;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        if (lane == 31) warp_sum[warp] = inc;
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t w = warp_sum[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= o) w += u;
+            }
+            warp_sum[lane] = w;
+        }
+        __syncthreads();
+        uint32_t e = base + inc - t + (warp ? warp_sum[warp - 1] : 0u);
+        base += warp_sum[31];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t i = at + 4 * tid + k;
+            if (i < n) counts[i] = e;
+            e += v[k];
+        }
+        __syncthreads();
+    }
+    if (tid == 0) counts[n] = base;
+}
+
+// one warp a segment: its pore voxels in order
+__global__ void pore_fill_kernel(const uint8_t* code, ListGrid g, const uint32_t* offs, uint32_t* idx, uint8_t* pcode) {
+    const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x & 31;
+    if (s >= g.nseg) return;
+    int xq0, y0, z;
+    segment_origin(g, s, xq0, y0, z);
+    uint32_t at = offs[s];
+    for (int k = lane; k < SEG_GROUPS; k += 32) {
+        const int xq = xq0 + k % LT_Q, y = y0 + k / LT_Q;
+        const uint32_t c = code4_at(code, xq, y, z, g.nx, g.ny, g.nz, g.cpitch);
+        const uint32_t n = (uint32_t)__popc(c & PORES);
+        uint32_t inc = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        uint32_t w = at + inc - n;
+        const uint32_t q = ((uint32_t)z * g.ny + y) * (uint32_t)g.pitch + 4u * xq;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t b = (c >> (8 * i)) & 127u;
+            if (b & CODE_PORE) {
+                idx[w] = q + i;
+                pcode[w++] = (uint8_t)b;
+            }
+        }
+        at += __shfl_sync(0xffffffffu, inc, 31);
+    }
+}
+
+// one CTA a chunk: the bounding box (x0, x1, y0, y1, z0, z1) of its entries
+__global__ void __launch_bounds__(128) chunk_box_kernel(const uint32_t* idx, uint32_t n, uint32_t chunks, FastDiv by_pitch,
+                                                        FastDiv by_ny, int pitch, int ny, int* box) {
+    __shared__ int lo[3], hi[3];
+    if (threadIdx.x < 3) {
+        lo[threadIdx.x] = 0x7fffffff;
+        hi[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    const uint32_t a = (uint32_t)((unsigned long long)n * blockIdx.x / chunks);
+    const uint32_t b = (uint32_t)((unsigned long long)n * (blockIdx.x + 1) / chunks);
+    int l[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, h[3] = {0, 0, 0};
+    for (uint32_t i = a + threadIdx.x; i < b; i += blockDim.x) {
+        const Cell v = cell_of(idx[i], by_pitch, by_ny, pitch, ny);
+        const int p[3] = {v.x, v.y, v.z};
+        for (int k = 0; k < 3; ++k) {
+            l[k] = min(l[k], p[k]);
+            h[k] = max(h[k], p[k] + 1);
+        }
+    }
+    for (int k = 0; k < 3; ++k) {
+        atomicMin(&lo[k], l[k]);
+        atomicMax(&hi[k], h[k]);
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        box[6 * blockIdx.x + 2 * threadIdx.x] = min(lo[threadIdx.x], hi[threadIdx.x]);
+        box[6 * blockIdx.x + 2 * threadIdx.x + 1] = hi[threadIdx.x];
+    }
+}
+
+// Raises *flag (host memory, read after the stream is synchronised) when a
+// solid voxel of a member's field holds anything but zero; with src, first
+// copies the dense arrays src[c] ([members][nz][ny][nx]) into the field.
+// One thread a group of four voxels.
+template <typename T>
+__global__ void field_in_kernel(T* field, const T* s0, const T* s1, const T* s2, const uint8_t* code, int nx, int ny,
+                                int nz, int pitch, int cpitch, long long comp, int members, int* flag) {
+    const int gq = pitch / 4;
+    const long long rows = (long long)ny * nz, n = rows * gq;
+    bool bad = false;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const long long row = q / gq;
+        const int x = 4 * (int)(q - row * gq);
+        const uint32_t c = *reinterpret_cast<const uint32_t*>(code + row * cpitch + x);
+        const long long dense = row * nx + x;
+        for (int b = 0; b < members; ++b) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                T* d = field + (3 * b + k) * comp + row * pitch + x;
+                const T* s = k == 0 ? s0 : k == 1 ? s1 : s2;
+                T v[4] = {0, 0, 0, 0};
+                if (s) {
+                    s += b * rows * nx + dense;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (x + i < nx) v[i] = s[i];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) d[i] = v[i];
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (x + i < nx) v[i] = d[i];
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) bad = bad || (!((c >> (8 * i)) & CODE_PORE) && !(v[i] == (T)0));
+            }
+        }
+    }
+    if (bad) *flag = 1;
+}
+
+// zero in the solid voxels of a field
+template <typename T>
+__global__ void solid_clear_kernel(T* field, const uint8_t* code, int nx, int ny, int nz, int pitch, int cpitch,
+                                   long long comp, int members) {
+    const int gq = pitch / 4;
+    const long long rows = (long long)ny * nz, n = rows * gq;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const long long row = q / gq;
+        const int x = 4 * (int)(q - row * gq);
+        const uint32_t c = *reinterpret_cast<const uint32_t*>(code + row * cpitch + x);
+        if ((c & PORES) == PORES) continue;
+        for (int k = 0; k < 3 * members; ++k) {
+            T* d = field + k * comp + row * pitch + x;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (!((c >> (8 * i)) & CODE_PORE)) d[i] = (T)0;
+        }
+    }
+}
+
+}  // namespace
+
+uint32_t list_segments(int nx, int ny, int nz) {
+    return (uint32_t)(((long long)nx + LT_X - 1) / LT_X * ((ny + LT_Y - 1) / LT_Y) * nz);
+}
+
+cudaError_t list_offsets(const uint8_t* code, int nx, int ny, int nz, int cpitch, bool groups, uint32_t* offs,
+                         cudaStream_t s) {
+    const ListGrid g{nx, ny, nz, 0, cpitch, (nx + LT_X - 1) / LT_X, list_segments(nx, ny, nz)};
+    list_count_kernel<<<(g.nseg + 7) / 8, 256, 0, s>>>(code, g, groups ? 1 : 0, offs);
+    list_scan_kernel<<<1, 1024, 0, s>>>(offs, g.nseg);
+    return cudaGetLastError();
+}
+
+cudaError_t fill_pore_list(const uint8_t* code, int nx, int ny, int nz, int pitch, int cpitch, const uint32_t* offs,
+                           uint32_t* idx, uint8_t* pcode, cudaStream_t s) {
+    const ListGrid g{nx, ny, nz, pitch, cpitch, (nx + LT_X - 1) / LT_X, list_segments(nx, ny, nz)};
+    pore_fill_kernel<<<(g.nseg + 7) / 8, 256, 0, s>>>(code, g, offs, idx, pcode);
+    return cudaGetLastError();
+}
+
+cudaError_t chunk_boxes(const uint32_t* idx, uint32_t n, uint32_t chunks, const FastDiv& by_pitch, const FastDiv& by_ny,
+                        int pitch, int ny, int* box, cudaStream_t s) {
+    chunk_box_kernel<<<chunks, 128, 0, s>>>(idx, n, chunks, by_pitch, by_ny, pitch, ny, box);
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t field_in(T* field, const T* const* src, const uint8_t* code, int nx, int ny, int nz, int pitch, int cpitch,
+                     long long comp, int members, int* flag, cudaStream_t s) {
+    const long long n = (long long)(pitch / 4) * ny * nz;
+    const int blocks = (int)std::min<long long>((n + 255) / 256, 152 * 8);
+    field_in_kernel<T><<<blocks, 256, 0, s>>>(field, src ? src[0] : nullptr, src ? src[1] : nullptr, src ? src[2] : nullptr,
+                                              code, nx, ny, nz, pitch, cpitch, comp, members, flag);
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t solid_clear(T* field, const uint8_t* code, int nx, int ny, int nz, int pitch, int cpitch, long long comp,
+                        int members, cudaStream_t s) {
+    const long long n = (long long)(pitch / 4) * ny * nz;
+    const int blocks = (int)std::min<long long>((n + 255) / 256, 152 * 8);
+    solid_clear_kernel<T><<<blocks, 256, 0, s>>>(field, code, nx, ny, nz, pitch, cpitch, comp, members);
+    return cudaGetLastError();
+}
+
+template cudaError_t field_in<float>(float*, const float* const*, const uint8_t*, int, int, int, int, int, long long, int,
+                                     int*, cudaStream_t);
+template cudaError_t field_in<double>(double*, const double* const*, const uint8_t*, int, int, int, int, int, long long,
+                                      int, int*, cudaStream_t);
+template cudaError_t solid_clear<float>(float*, const uint8_t*, int, int, int, int, int, long long, int, cudaStream_t);
+template cudaError_t solid_clear<double>(double*, const uint8_t*, int, int, int, int, int, long long, int, cudaStream_t);
+
+}  // namespace bt

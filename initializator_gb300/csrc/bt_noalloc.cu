@@ -174,6 +174,9 @@ void fill(const bt_config& c, bt::StepParams<T>& P, const void* const in[3], voi
         P.an[k] = (T)an[k];
         P.peqn[k] = (T)(c.p_eq * an[k]);
     }
+    P.axis = -1;
+    for (int k = 0; k < 3; ++k)
+        if (an[k] == 1.0 && an[(k + 1) % 3] == 0.0 && an[(k + 2) % 3] == 0.0) P.axis = k;
     P.b = (T)(dTime * c.gamma);
     P.dx = (T)c.dx; P.dy = (T)c.dy; P.dz = (T)c.dz;
     const double D = c.d_pore;

@@ -26,6 +26,7 @@
 // of steps without host involvement.
 #pragma once
 #include <cmath>
+#include <cstdlib>
 #include "bt_internal.h"
 
 namespace bt {
@@ -33,6 +34,23 @@ namespace bt {
 constexpr int SCHEME_REF = 0;
 constexpr int SCHEME_KSPACE = 1;
 constexpr int ZCHUNK_MAX = 1024;
+
+// programmatic dependent launch: a kernel overlaps its step-independent
+// prologue with the previous launch's tail (BT_NO_PDL turns it off)
+static inline cudaLaunchConfig_t pdl_config(dim3 grid, dim3 block, int smem, cudaStream_t s,
+                                            cudaLaunchAttribute* attr) {
+    static const bool pdl = std::getenv("BT_NO_PDL") == nullptr;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cfg;
+}
 
 template <typename T>
 struct Acc;
@@ -58,6 +76,17 @@ struct Acc<double> {
 // velocity, 1 otherwise (1e-50 underflows in FP32, so FP32 tests v != 0).
 __device__ __forceinline__ float upsw(float v) { return v != 0.f ? 1.f : 0.f; }
 __device__ __forceinline__ double upsw(double v) { return v / (v + 1.0e-50); }
+
+// A face velocity whose switch is known without the division: zero (switch
+// v / 1e-50 = v = 0), or finite and at least 2^-111 (3.9e-34) in size, where
+// half an ulp exceeds 1e-50, so that v + 1e-50 rounds to v and the switch is
+// exactly 1.
+__device__ __forceinline__ bool upsw_plain(double v) {
+    const int hi = __double2hiint(v) & 0x7fffffff;
+    return (hi >= 0x39000000 && hi < 0x7ff00000) || (hi | __double2loint(v)) == 0;
+}
+// not finite (exponent all ones)
+__device__ __forceinline__ bool not_finite(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
 
 // OrtTransform (cpp:2536-2550) with the angle's cosine c and sine s given
 __device__ __forceinline__ void ort_cs(double& x, double& y, double& z, double nx, double ny, double nz, double c,
@@ -301,6 +330,7 @@ __device__ __forceinline__ void reduce_partials(const StepParams<T>& P, long lon
     if (threadIdx.x + blockDim.x * threadIdx.y == 0) {
         P.ctl->ticket = 0;
         P.ctl->step = step + 1;
+        P.ctl->gen_from = step + 1;
         __threadfence();
     }
 }
@@ -408,6 +438,146 @@ __global__ void __launch_bounds__(256) step_finish_kernel(const __grid_constant_
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const long long step = __ldcg(&P.ctl->fstep[1 - P.side]) - 1;
     reduce_partials<T>(P, step, nb_per, red);
+}
+
+// The new value o of one pore voxel before the step's pulses: relaxation
+// toward p_eq n, precession (bb = dTime g B_noise), upwind advection and
+// harmonic-mean diffusion (ExplicitSimple, cpp:3162-3263). nb[c][q] and vf[q],
+// df[q]: the neighbours, face velocities and face diffusivities -x +x -y +y
+// -z +z (KSPACE: neighbours already in the voxel's frame). In double precision
+// every product and sum is the reference's, in its order; WHOLE forms all of
+// them.
+template <typename T, int SCHEME, bool VEL, bool PREC>
+__device__ __noinline__ void voxel_step_whole(const StepParams<T>& P, const T (&p0)[3], const T (&nb)[3][6], T dtt1,
+                                              T dtt2, const T (&vf)[6], const T (&df)[6], const T (&bb)[3], T (&o)[3]);
+
+template <typename T, int SCHEME, bool VEL, bool PREC, bool WHOLE>
+__device__ __forceinline__ void voxel_step_form(const StepParams<T>& P, const T (&p0)[3], const T (&nb)[3][6], T dtt1,
+                                                T dtt2, const T (&vf)[6], const T (&df)[6], const T (&bb)[3], T (&o)[3]) {
+    const T px0 = p0[0], py0 = p0[1], pz0 = p0[2];
+    T r[3];
+    if constexpr (SCHEME == SCHEME_REF) {
+        if (!WHOLE && P.axis >= 0) {
+            // n along an axis: n (n.M) is that component
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                r[c] = P.axis == c ? p0[c] + dtt1 * (P.peqn[c] - p0[c]) : p0[c] - dtt2 * p0[c];
+        } else {
+            const T div = P.an[0] * px0 + P.an[1] * py0 + P.an[2] * pz0;
+            const T divx = P.an[0] * div, divy = P.an[1] * div, divz = P.an[2] * div;
+            r[0] = px0 + dtt1 * (P.peqn[0] - divx) + dtt2 * (divx - px0);
+            r[1] = py0 + dtt1 * (P.peqn[1] - divy) + dtt2 * (divy - py0);
+            r[2] = pz0 + dtt1 * (P.peqn[2] - divz) + dtt2 * (divz - pz0);
+        }
+        if constexpr (PREC) {
+            r[0] += (T)0.0 - bb[1] * pz0 + bb[2] * py0;
+            r[1] += (T)0.0 + bb[0] * pz0 - bb[2] * px0;
+            r[2] += (T)0.0 - bb[0] * py0 + bb[1] * px0;
+        }
+    } else {
+        // B0 along z: the reference relaxation with n = (0, 0, 1)
+        r[0] = px0 + dtt2 * ((T)0.0 - px0);
+        r[1] = py0 + dtt2 * ((T)0.0 - py0);
+        r[2] = pz0 + dtt1 * (P.peqn[2] - pz0);
+        if constexpr (WHOLE) r[2] += dtt2 * (pz0 - pz0);
+    }
+    auto diffuse = [&](T a, int c) {
+        return a + (P.hxx * (df[1] * (nb[c][1] - p0[c]) - df[0] * (p0[c] - nb[c][0])) +
+                    P.hyy * (df[3] * (nb[c][3] - p0[c]) - df[2] * (p0[c] - nb[c][2])) +
+                    P.hzz * (df[5] * (nb[c][5] - p0[c]) - df[4] * (p0[c] - nb[c][4])));
+    };
+    if constexpr (!VEL) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) o[c] = P.diffusion ? diffuse(r[c], c) : r[c];
+    } else {
+        const T hx2 = (T)0.5 * P.hx, hy2 = (T)0.5 * P.hy, hz2 = (T)0.5 * P.hz;
+        if constexpr (!WHOLE) {
+            // u + |u| (u - |u| for u < 0) = 2 u = the two faces' sum, gated by
+            // the face it draws from
+            T w[3];
+            bool up[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const T s = vf[2 * a] + vf[2 * a + 1];
+                up[a] = s > (T)0.0;
+                w[a] = (up[a] ? vf[2 * a] : vf[2 * a + 1]) != (T)0.0 ? s : (T)0.0;
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const T dx = up[0] ? p0[c] - nb[c][0] : nb[c][1] - p0[c];
+                const T dy = up[1] ? p0[c] - nb[c][2] : nb[c][3] - p0[c];
+                const T dz = up[2] ? p0[c] - nb[c][4] : nb[c][5] - p0[c];
+                o[c] = diffuse(r[c] - (hx2 * (w[0] * dx) + hy2 * (w[1] * dy) + hz2 * (w[2] * dz)), c);
+            }
+        } else {
+            const T um = vf[0], up = vf[1], vm = vf[2], vp = vf[3], wlo = vf[4], whi = vf[5];
+            const T upp = upsw(up), umm = upsw(um), vpp = upsw(vp), vmm = upsw(vm);
+            const T wpp = upsw(whi), wmm = upsw(wlo);
+            const T u = (T)0.5 * (um + up), v = (T)0.5 * (vm + vp), w = (T)0.5 * (wlo + whi);
+            const T ud = fabs(u), vd = fabs(v), wd = fabs(w);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                T a = r[c];
+                a -= hx2 * ((u - ud) * (nb[c][1] - p0[c]) * upp + (u + ud) * (p0[c] - nb[c][0]) * umm) +
+                     hy2 * ((v - vd) * (nb[c][3] - p0[c]) * vpp + (v + vd) * (p0[c] - nb[c][2]) * vmm) +
+                     hz2 * ((w - wd) * (nb[c][5] - p0[c]) * wpp + (w + wd) * (p0[c] - nb[c][4]) * wmm);
+                o[c] = P.diffusion ? diffuse(a, c) : a;
+            }
+        }
+    }
+}
+
+template <typename T, int SCHEME, bool VEL, bool PREC>
+__device__ __noinline__ void voxel_step_whole(const StepParams<T>& P, const T (&p0)[3], const T (&nb)[3][6], T dtt1,
+                                              T dtt2, const T (&vf)[6], const T (&df)[6], const T (&bb)[3], T (&o)[3]) {
+    voxel_step_form<T, SCHEME, VEL, PREC, true>(P, p0, nb, dtt1, dtt2, vf, df, bb, o);
+}
+
+// FP64: GB300 issues two FP64 lanes a cycle and SM, so operations whose result
+// is known are left out: of the two halves of an axis' upwind difference one
+// carries the factor u - |u| or u + |u| = 0 and the switch of the other is
+// almost always exactly 1 (six divisions a voxel); n along an axis makes most
+// products of the relaxation 0. What is left out adds zero, so the sums are the
+// same numbers as the whole form's for finite fields; a voxel whose switches
+// cannot be told, whose result is not finite, or a handle without diffusion
+// (where a neighbour that is not finite could go unseen) takes the whole form.
+// ~230 FP64 operations a voxel with flow become ~105, ~92 without become ~73.
+template <typename T, int SCHEME, bool VEL, bool PREC>
+__device__ __forceinline__ void voxel_step(const StepParams<T>& P, const T (&p0)[3], const T (&nb)[3][6], T dtt1, T dtt2,
+                                           const T (&vf)[6], const T (&df)[6], const T (&bb)[3], T (&o)[3]) {
+    if constexpr (sizeof(T) == 4) {
+        voxel_step_form<T, SCHEME, VEL, PREC, true>(P, p0, nb, dtt1, dtt2, vf, df, bb, o);
+    } else {
+        bool plain = true;
+        if constexpr (VEL) {
+            plain = P.diffusion != 0;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) plain = plain && upsw_plain(vf[q]);
+        }
+        if (plain) {
+            voxel_step_form<T, SCHEME, VEL, PREC, false>(P, p0, nb, dtt1, dtt2, vf, df, bb, o);
+            plain = !not_finite(o[0]) && !not_finite(o[1]) && !not_finite(o[2]);
+        }
+        if (!plain) {
+            // copies, so that the arrays themselves stay in registers
+            T p0c[3], nbc[3][6], vfc[6], dfc[6], bbc[3], oc[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                p0c[c] = p0[c];
+                bbc[c] = bb[c];
+#pragma unroll
+                for (int q = 0; q < 6; ++q) nbc[c][q] = nb[c][q];
+            }
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                vfc[q] = vf[q];
+                dfc[q] = df[q];
+            }
+            voxel_step_whole<T, SCHEME, VEL, PREC>(P, p0c, nbc, dtt1, dtt2, vfc, dfc, bbc, oc);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) o[c] = oc[c];
+        }
+    }
 }
 
 template <typename T, int SCHEME, bool VEL, bool PREC>
@@ -583,69 +753,21 @@ __global__ void __launch_bounds__(NTHREADS) step_kernel(const __grid_constant__ 
                         nb[1][q] = open[q] ? ph[q][0] * im + ph[q][1] * re : py0;
                     }
                 }
-                T ax, ay, az;
-                if constexpr (SCHEME == SCHEME_REF) {
-                    const T div = P.an[0] * px0 + P.an[1] * py0 + P.an[2] * pz0;
-                    const T divx = P.an[0] * div, divy = P.an[1] * div, divz = P.an[2] * div;
-                    ax = px0 + dtt1 * (P.peqn[0] - divx) + dtt2 * (divx - px0);
-                    ay = py0 + dtt1 * (P.peqn[1] - divy) + dtt2 * (divy - py0);
-                    az = pz0 + dtt1 * (P.peqn[2] - divz) + dtt2 * (divz - pz0);
-                    if constexpr (PREC) {
-                        const T bbxb = P.b * (gdx * ((T)x + (T)0.5));
-                        const T bbyb = P.b * (gdy * ((T)y + (T)0.5));
-                        const T bbzb = P.b * (gdz * ((T)z + (T)0.5));
-                        ax += (T)0.0 - bbyb * pz0 + bbzb * py0;
-                        ay += (T)0.0 + bbxb * pz0 - bbzb * px0;
-                        az += (T)0.0 - bbxb * py0 + bbyb * px0;
-                    }
-                } else {
-                    // B0 along z: the reference relaxation with n = (0, 0, 1)
-                    ax = px0 + dtt2 * ((T)0.0 - px0);
-                    ay = py0 + dtt2 * ((T)0.0 - py0);
-                    az = pz0 + dtt1 * (P.peqn[2] - pz0) + dtt2 * (pz0 - pz0);
-                }
-                if constexpr (VEL) {
-                    const T upp = upsw(up), umm = upsw(um), vpp = upsw(vp), vmm = upsw(vm);
-                    const T wpp = upsw(whi), wmm = upsw(wlo);
-                    const T u = (T)0.5 * (um + up), v = (T)0.5 * (vm + vp), w = (T)0.5 * (wlo + whi);
-                    const T ud = fabs(u), vd = fabs(v), wd = fabs(w);
-                    const T hx2 = (T)0.5 * P.hx, hy2 = (T)0.5 * P.hy, hz2 = (T)0.5 * P.hz;
-                    const T p0[3] = {px0, py0, pz0};
-                    T a[3] = {ax, ay, az};
+                T dfq[6];
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        a[c] -= hx2 * ((u - ud) * (nb[c][1] - p0[c]) * upp + (u + ud) * (p0[c] - nb[c][0]) * umm) +
-                                hy2 * ((v - vd) * (nb[c][3] - p0[c]) * vpp + (v + vd) * (p0[c] - nb[c][2]) * vmm) +
-                                hz2 * ((w - wd) * (nb[c][5] - p0[c]) * wpp + (w + wd) * (p0[c] - nb[c][4]) * wmm);
-                    }
-                    ax = a[0];
-                    ay = a[1];
-                    az = a[2];
+                for (int q = 0; q < 6; ++q)
+                    dfq[q] = P.fw ? P.fw[q * P.fstride + vox] : (f & (1 << q)) ? P.dps : P.dpp;
+                const T p0[3] = {px0, py0, pz0};
+                const T vf[6] = {um, up, vm, vp, wlo, whi};
+                T bb[3] = {0, 0, 0};
+                if constexpr (PREC && SCHEME == SCHEME_REF) {
+                    bb[0] = P.b * (gdx * ((T)x + (T)0.5));
+                    bb[1] = P.b * (gdy * ((T)y + (T)0.5));
+                    bb[2] = P.b * (gdz * ((T)z + (T)0.5));
                 }
-                if (P.diffusion) {
-                    T dxm = (f & 1) ? P.dps : P.dpp, dxp = (f & 2) ? P.dps : P.dpp;
-                    T dym = (f & 4) ? P.dps : P.dpp, dyp = (f & 8) ? P.dps : P.dpp;
-                    T dzm = (f & 16) ? P.dps : P.dpp, dzp = (f & 32) ? P.dps : P.dpp;
-                    if (P.fw) {
-                        dxm = P.fw[vox];
-                        dxp = P.fw[P.fstride + vox];
-                        dym = P.fw[2 * P.fstride + vox];
-                        dyp = P.fw[3 * P.fstride + vox];
-                        dzm = P.fw[4 * P.fstride + vox];
-                        dzp = P.fw[5 * P.fstride + vox];
-                    }
-                    const T p0[3] = {px0, py0, pz0};
-                    T a[3] = {ax, ay, az};
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        a[c] += P.hxx * (dxp * (nb[c][1] - p0[c]) - dxm * (p0[c] - nb[c][0])) +
-                                P.hyy * (dyp * (nb[c][3] - p0[c]) - dym * (p0[c] - nb[c][2])) +
-                                P.hzz * (dzp * (nb[c][5] - p0[c]) - dzm * (p0[c] - nb[c][4]));
-                    }
-                    ax = a[0];
-                    ay = a[1];
-                    az = a[2];
-                }
+                T oc[3];
+                voxel_step<T, SCHEME, VEL, PREC>(P, p0, nb, dtt1, dtt2, vf, dfq, bb, oc);
+                T ax = oc[0], ay = oc[1], az = oc[2];
                 T lx = ax, ly = ay;  // lab-frame transverse components
                 T er = 1, ei = 0;
                 if constexpr (SCHEME == SCHEME_KSPACE) {

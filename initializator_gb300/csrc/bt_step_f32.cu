@@ -4,6 +4,7 @@
 
 #include "bt_step_tma.cuh"
 #include "bt_step_mac.cuh"
+#include "bt_step_pore.cuh"
 
 namespace bt {
 
@@ -23,6 +24,22 @@ cudaError_t launch_sums<float>(const StepParams<float>& p, double* kvec_and_grid
 template <>
 cudaError_t launch_mac<float>(const StepParams<float>& p, float* const pred[3], int vel, int prec, dim3 grid, cudaStream_t s) {
     return launch_mac_impl<float>(p, pred, vel, prec, grid, s);
+}
+
+template <>
+cudaError_t launch_step_list<float>(const StepParams<float>& p, int scheme, int vel, int prec, cudaStream_t s) {
+    return p.phw ? launch_step_list_impl<float, true>(p, scheme, vel, prec, s)
+                 : launch_step_list_impl<float, false>(p, scheme, vel, prec, s);
+}
+
+template <>
+cudaError_t launch_mac_list<float>(const StepParams<float>& p, float* const pred[3], int vel, int prec, cudaStream_t s) {
+    return launch_mac_list_impl<float>(p, pred, vel, prec, s);
+}
+
+template <>
+cudaError_t launch_list_finish<float>(const StepParams<float>& p, cudaStream_t s) {
+    return launch_list_finish_impl<float>(p, s);
 }
 
 template <>

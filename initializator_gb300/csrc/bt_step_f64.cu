@@ -3,6 +3,7 @@
 // keeps the reference's rounding step for step.
 #include "bt_step.cuh"
 #include "bt_step_mac.cuh"
+#include "bt_step_pore.cuh"
 
 namespace bt {
 
@@ -22,6 +23,22 @@ cudaError_t launch_sums<double>(const StepParams<double>& p, double* kvec_and_gr
 template <>
 cudaError_t launch_mac<double>(const StepParams<double>& p, double* const pred[3], int vel, int prec, dim3 grid, cudaStream_t s) {
     return launch_mac_impl<double>(p, pred, vel, prec, grid, s);
+}
+
+template <>
+cudaError_t launch_step_list<double>(const StepParams<double>& p, int scheme, int vel, int prec, cudaStream_t s) {
+    return p.phw ? launch_step_list_impl<double, true>(p, scheme, vel, prec, s)
+                 : launch_step_list_impl<double, false>(p, scheme, vel, prec, s);
+}
+
+template <>
+cudaError_t launch_mac_list<double>(const StepParams<double>& p, double* const pred[3], int vel, int prec, cudaStream_t s) {
+    return launch_mac_list_impl<double>(p, pred, vel, prec, s);
+}
+
+template <>
+cudaError_t launch_list_finish<double>(const StepParams<double>& p, cudaStream_t s) {
+    return launch_list_finish_impl<double>(p, s);
 }
 
 template <>

@@ -1,0 +1,628 @@
+// Generic step kernels over the pore list: one thread per pore voxel.
+//
+// What bounds them: FP64 fields are bound by the FP64 pipe (two lanes a cycle
+// and SM on GB300: ~95 operations a voxel without flow, ~125 with). A dense
+// z-march (step_kernel, bt_step.cuh) issues each of them for whole rows of 32
+// voxels, solid lanes included, since nearly every row of a rock holds a pore
+// voxel; the list fills every lane with a pore voxel. The neighbours are read
+// straight from global memory: in list order (bt_list.cuh) they sit in L1, and
+// two dozen independent loads a thread need no staging or barriers.
+// FP32 fields (per-voxel rates, positional pulses) gain by the same token what
+// the dense march spent on its two barriers a plane.
+//
+// Measured per time step, dense march before -> list (GB300, launches and sums
+// included): FP64 64^3 sphere pack (65 % pore), no flow, 77 -> 39 us (~25 us of
+// FP64 issue); FP64 MacCormack 90 x 75 x 66 with flow and a gradient 450 ->
+// 210 us; FP32 128 x 112 x 96 with per-voxel rates, flow and the two-component
+// sums 163 -> 39 us (the sums were two launches of their own, in FP64).
+// 4 (FP64) or 5 (FP32) resident CTAs of 128 threads a SM: one CTA a 128-entry
+// chunk instead took 52 us for the first and left a last wave nearly empty.
+//
+// The arithmetic is voxel_step's (bt_step.cuh), the FP64 field bit for bit the
+// dense kernel's; the solid voxels of the output are not written (they hold
+// zero, bt_list.cuh).
+#pragma once
+#include "bt_list.cuh"
+#include "bt_step.cuh"
+
+namespace bt {
+
+constexpr int PT = 128;  // threads of a CTA of the list kernels
+static_assert(PT == LIST_THREADS, "bt_list.cuh");
+
+// running sums of one thread in float-float (FP32 fields): s + l
+struct Acc2 {
+    float s = 0.f, l = 0.f;
+    // + a * w exactly
+    __device__ __forceinline__ void add_product(float a, float w) {
+        const float p = a * w;
+        const float pe = fmaf(a, w, -p);
+        float t, e;
+        two_sum(s, p, t, e);
+        s = t;
+        l += e + pe;
+    }
+};
+
+// The CTA's NS sums (thread t's value c in sm[c][t], FP64 or float-float), each
+// added by one warp in a fixed order, to the chunk's slot of this input side's
+// partials (sums 3.. to part6). One warp a sum takes 8 dependent FP64 additions
+// instead of 15 in every warp.
+template <typename T, int NS>
+__device__ __forceinline__ void chunk_sums(const StepParams<T>& P, unsigned b, unsigned chunk, double (*sm)[PT]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();
+    for (int c = warp; c < NS; c += PT / 32) {
+        double t;
+        if constexpr (sizeof(T) == 8) {
+            t = (sm[c][lane] + sm[c][lane + 32]) + (sm[c][lane + 64] + sm[c][lane + 96]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        } else {
+            const float2* p = reinterpret_cast<const float2*>(sm[c]);
+            float h = p[lane].x, l = p[lane].y;
+#pragma unroll
+            for (int k = 1; k < PT / 32; ++k) {
+                float s, e;
+                two_sum(h, p[lane + 32 * k].x, s, e);
+                h = s;
+                l += e + p[lane + 32 * k].y;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float bh = __shfl_down_sync(0xffffffffu, h, o), bl = __shfl_down_sync(0xffffffffu, l, o);
+                float s, e;
+                two_sum(h, bh, s, e);
+                e += l + bl;
+                h = s + e;
+                l = e - (h - s);
+            }
+            t = (double)h + (double)l;
+        }
+        if (lane == 0) {
+            if (c < 3) P.partials[3ull * ((unsigned long long)b * P.pchunks + chunk) + c] = t;
+            else P.part6[6ull * chunk + (c - 3)] = t;
+        }
+    }
+}
+
+// One CTA: the sums of `step` of batch member b from its chunks' partials, in a
+// fixed order, into M(t) (and the two-component sums), with the NaN/Inf check.
+template <typename T, int NS>
+__device__ __forceinline__ void add_partials(const StepParams<T>& P, const double* parts, const double* parts6, unsigned b,
+                                             long long step, double (*sm)[PT]) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned nb = P.nbatch > 1 ? (unsigned)P.nbatch : 1u;
+    double t[NS] = {};
+#pragma unroll 4
+    for (unsigned q = tid; q < P.pchunks; q += PT) {
+#pragma unroll
+        for (int c = 0; c < NS; ++c)
+            t[c] += c < 3 ? __ldcg(&parts[3ull * ((unsigned long long)b * P.pchunks + q) + c])
+                          : __ldcg(&parts6[6ull * q + (c - 3)]);
+    }
+#pragma unroll
+    for (int c = 0; c < NS; ++c) sm[c][tid] = t[c];
+    __syncthreads();
+    const long long slot = step - __ldcg(&P.ctl->mt_base);
+    for (int c = warp; c < NS; c += PT / 32) {
+        double u = (sm[c][lane] + sm[c][lane + 32]) + (sm[c][lane + 64] + sm[c][lane + 96]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) u += __shfl_down_sync(0xffffffffu, u, o);
+        if (lane == 0) {
+            if (c < 3 && slot >= 0 && slot < P.mt_cap) P.mt[3 * (slot * nb + b) + c] = u;
+            else if (c >= 3 && slot >= 0 && slot < P.mt6_cap) P.mt6[6 * slot + (c - 3)] = u;
+            else atomicOr(&P.ctl->status, 1);
+            if (c < 3 && !isfinite(u)) atomicOr(&P.ctl->status, 4);
+        }
+    }
+}
+
+// closes a run of list steps: the last step's sums (one CTA a member), the step
+// counters
+template <typename T, int NS>
+__global__ void __launch_bounds__(PT) list_finish_kernel(const __grid_constant__ StepParams<T> P) {
+    __shared__ double sums[NS][PT];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const long long end = __ldcg(&P.ctl->fstep[1 - P.side]);
+    add_partials<T, NS>(P, P.partials, P.part6, blockIdx.x, end - 1, sums);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        P.ctl->step = end;
+        P.ctl->fstep[P.side] = end;
+        P.ctl->gen_from = end;
+    }
+}
+
+// This CTA's chunk of the list (even shares) and batch member; members of a
+// chunk are neighbouring CTAs, so the geometry they share comes from L2. The
+// launch's first CTA of each member (adder) has no chunk: it adds the previous
+// step's partials, off the other CTAs' path.
+struct Chunk {
+    unsigned b, c;
+    bool adder;
+    uint32_t first, last;
+};
+__device__ __forceinline__ Chunk chunk_of(uint32_t n, uint32_t chunks, int nbatch) {
+    Chunk k;
+    const unsigned nb = nbatch > 1 ? (unsigned)nbatch : 1u;
+    k.b = blockIdx.x % nb;
+    k.adder = blockIdx.x < nb;
+    k.c = k.adder ? 0u : blockIdx.x / nb - 1u;
+    k.first = (uint32_t)((unsigned long long)n * k.c / chunks);
+    k.last = (uint32_t)((unsigned long long)n * (k.c + 1) / chunks);
+    return k;
+}
+
+// the six neighbours of element q of the components in[], copy ghosts (the
+// voxel itself) on domain faces; open[f]: the face lies inside the domain
+template <typename T>
+__device__ __forceinline__ void load_neighbours(const T* const (&in)[3], uint32_t q, const bool (&open)[6], int pitch,
+                                                long long plane, T (&p0)[3], T (&nb)[3][6]) {
+    const long long o[6] = {open[0] ? (long long)q - 1 : q,     open[1] ? (long long)q + 1 : q,
+                            open[2] ? (long long)q - pitch : q, open[3] ? (long long)q + pitch : q,
+                            open[4] ? (long long)q - plane : q, open[5] ? (long long)q + plane : q};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        p0[c] = in[c][q];
+#pragma unroll
+        for (int f = 0; f < 6; ++f) nb[c][f] = in[c][o[f]];
+    }
+}
+
+// offsets of the far edge cells of cell (x, y, z) (periodic faces)
+__device__ __forceinline__ void far_cells(const Cell& v, int nx, int ny, int nz, int pitch, long long plane,
+                                          long long (&far)[6]) {
+    const long long row = (long long)v.z * plane + (long long)v.y * pitch;
+    far[0] = row + nx - 1;
+    far[1] = row;
+    far[2] = (long long)v.z * plane + (long long)(ny - 1) * pitch + v.x;
+    far[3] = (long long)v.z * plane + v.x;
+    far[4] = (long long)(nz - 1) * plane + (long long)v.y * pitch + v.x;
+    far[5] = (long long)v.y * pitch + v.x;
+}
+
+template <typename T, int SCHEME, bool VEL, bool PREC, bool PHS>
+__global__ void __launch_bounds__(PT, list_ctas_per_sm(sizeof(T))) pore_step_kernel(const __grid_constant__ StepParams<T> P) {
+    constexpr int NS = PHS ? 9 : 3;
+    __shared__ double sums[NS][PT];
+    __shared__ PulsePrep pprep;
+    // KSPACE: lab-frame phase factors over this chunk's bounding box
+    extern __shared__ __align__(16) unsigned char phase_raw[];
+    T(*ex)[2] = reinterpret_cast<T(*)[2]>(phase_raw);
+
+    const int tid = threadIdx.x;
+    const int nx = P.nx, ny = P.ny, nz = P.nz, pitch = P.pitch;
+    const long long plane = P.plane;
+    const Chunk k = chunk_of(P.npore, P.pchunks, P.nbatch);
+    const unsigned nbt = P.nbatch > 1 ? (unsigned)P.nbatch : 1u;
+    // the next launch's CTAs may become resident; they wait below until this
+    // grid has completed
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const long long step = __ldcg(&P.ctl->fstep[P.side]);
+    if (k.adder) {
+        if (k.b == 0 && tid == 0) P.ctl->fstep[1 - P.side] = step + 1;
+        if (step > __ldcg(&P.ctl->gen_from)) add_partials<T, NS>(P, P.partials_prev, P.part6_prev, k.b, step - 1, sums);
+        return;
+    }
+    const StepInfo* si = P.steps + (step < P.nsched ? step : P.nsched) * nbt + k.b;
+    const T* in[3] = {P.in[0] + k.b * P.bstride, P.in[1] + k.b * P.bstride, P.in[2] + k.b * P.bstride};
+    T* out[3] = {P.out[0] + k.b * P.bstride, P.out[1] + k.b * P.bstride, P.out[2] + k.b * P.bstride};
+
+    T gd[3] = {0, 0, 0};
+    if constexpr (PREC && SCHEME == SCHEME_REF) {
+        gd[0] = (T)(si->grad[0] * P.dxd);
+        gd[1] = (T)(si->grad[1] * P.dyd);
+        gd[2] = (T)(si->grad[2] * P.dzd);
+    }
+    T ph[6][2];
+    int bx0 = 0, by0 = 0, bz0 = 0, lx = 0, ly = 0;
+    if constexpr (SCHEME == SCHEME_KSPACE) {
+#pragma unroll
+        for (int f = 0; f < 6; ++f) {
+            ph[f][0] = (T)si->phase[f][0];
+            ph[f][1] = (T)si->phase[f][1];
+        }
+        const int* bo = P.pbox + 6 * k.c;
+        bx0 = bo[0];
+        by0 = bo[2];
+        bz0 = bo[4];
+        lx = bo[1] - bx0;
+        ly = bo[3] - by0;
+        const int lz = bo[5] - bz0;
+        for (int q = tid; q < lx; q += PT) lab_phase<T>(si->knext[0], bx0 + q, P.dxd, ex[q][0], ex[q][1]);
+        for (int q = tid; q < ly; q += PT) lab_phase<T>(si->knext[1], by0 + q, P.dyd, ex[lx + q][0], ex[lx + q][1]);
+        for (int q = tid; q < lz; q += PT)
+            lab_phase<T>(si->knext[2], bz0 + q, P.dzd, ex[lx + ly + q][0], ex[lx + ly + q][1]);
+        __syncthreads();
+    }
+    const int npulse = si->pulse_count;
+    const DevPulse* pulses = P.pulses + si->pulse_first;
+    if (npulse) {  // CTA-uniform
+        pulse_prep(pprep, pulses, npulse, tid);
+        __syncthreads();
+    }
+    // non-copy domain faces take their own ghosts from the second step on (the
+    // first step of a run from step 0 reads the reference's initial copies)
+    const int bcs[3] = {P.bc[0], P.bc[1], P.bc[2]};
+    const bool bc_live = (bcs[0] | bcs[1] | bcs[2]) != 0 && step > 0;
+
+    Acc<T> acc[3];
+    Acc2 acc6f[PHS ? 6 : 1];
+    double acc6[PHS ? 6 : 1] = {};
+
+    for (uint32_t i = k.first + tid; i < k.last; i += PT) {
+        const uint32_t q = P.pidx[i];
+        const int f = P.pcode[i] & 63;
+        const Cell v = cell_of(q, P.by_pitch, P.by_ny, pitch, ny);
+        bool open[6] = {v.x > 0, v.x < nx - 1, v.y > 0, v.y < ny - 1, v.z > 0, v.z < nz - 1};
+        T p0[3], nb[3][6];
+        load_neighbours<T>(in, q, open, pitch, plane, p0, nb);
+        T vf[6] = {0, 0, 0, 0, 0, 0};
+        if constexpr (VEL) {
+            const T* vx = P.vx + ((long long)v.z * ny + v.y) * P.vxpitch + v.x;
+            const T* vy = P.vy + ((long long)v.z * (ny + 1) + v.y) * pitch + v.x;
+            vf[0] = vx[0];
+            vf[1] = vx[1];
+            vf[2] = vy[0];
+            vf[3] = vy[pitch];
+            vf[4] = P.vz[q];
+            vf[5] = P.vz[q + plane];
+        }
+        T dtt1 = P.fdtt ? P.fdtt[q] : P.dtt1[f], dtt2 = P.fdtt ? P.fdtt[P.fstride + q] : P.dtt2[f];
+        if (P.pal) {
+            // FP32 per-voxel rates through the rate palette
+            const int id = P.pal_idx[((long long)v.z * ny + v.y) * P.cpitch + v.x];
+            dtt1 = (T)P.pal[2 * id];
+            dtt2 = (T)P.pal[2 * id + 1];
+        }
+        T df[6];
+#pragma unroll
+        for (int a = 0; a < 6; ++a) df[a] = P.fw ? P.fw[a * P.fstride + q] : (f & (1 << a)) ? P.dps : P.dpp;
+        T w1 = 0, w2 = 0;
+        if constexpr (PHS) {
+            w1 = P.phw[q];
+            w2 = P.phw[P.fstride + q];
+        }
+        if (bc_live) {
+            long long far[6];
+            far_cells(v, nx, ny, nz, pitch, plane, far);
+            face_ghosts<T, SCHEME>(bcs, si, in, far, nb, open);
+        }
+        if constexpr (SCHEME == SCHEME_KSPACE) {
+            // transverse neighbours in the frame of this voxel; the voxel
+            // itself on a copy face (zero difference)
+#pragma unroll
+            for (int a = 0; a < 6; ++a) {
+                const T re = nb[0][a], im = nb[1][a];
+                nb[0][a] = open[a] ? ph[a][0] * re - ph[a][1] * im : p0[0];
+                nb[1][a] = open[a] ? ph[a][0] * im + ph[a][1] * re : p0[1];
+            }
+        }
+        T bb[3] = {0, 0, 0};
+        if constexpr (PREC && SCHEME == SCHEME_REF) {
+            bb[0] = P.b * (gd[0] * ((T)v.x + (T)0.5));
+            bb[1] = P.b * (gd[1] * ((T)v.y + (T)0.5));
+            bb[2] = P.b * (gd[2] * ((T)v.z + (T)0.5));
+        }
+        T o[3];
+        voxel_step<T, SCHEME, VEL, PREC>(P, p0, nb, dtt1, dtt2, vf, df, bb, o);
+        T lr = o[0], li = o[1];  // lab-frame transverse components
+        if constexpr (SCHEME == SCHEME_KSPACE) {
+            const T exr = ex[v.x - bx0][0], exi = ex[v.x - bx0][1];
+            const T eyr = ex[lx + v.y - by0][0], eyi = ex[lx + v.y - by0][1];
+            const T ezr = ex[lx + ly + v.z - bz0][0], ezi = ex[lx + ly + v.z - bz0][1];
+            const T xyr = exr * eyr - exi * eyi, xyi = exr * eyi + exi * eyr;
+            const T er = xyr * ezr - xyi * ezi, ei = xyr * ezi + xyi * ezr;
+            lr = er * o[0] - ei * o[1];
+            li = er * o[1] + ei * o[0];
+            if (npulse) {
+                apply_pulses<T>(pprep, pulses, npulse, lr, li, o[2], v.x, v.y, v.z, P.dxd, P.dyd, P.dzd, P.gamma, nx, ny,
+                                nz);
+                o[0] = er * lr + ei * li;  // back to the frame: conj(e) * lab
+                o[1] = er * li - ei * lr;
+            }
+        } else if (npulse) {
+            apply_pulses<T>(pprep, pulses, npulse, lr, li, o[2], v.x, v.y, v.z, P.dxd, P.dyd, P.dzd, P.gamma, nx, ny, nz);
+            o[0] = lr;
+            o[1] = li;
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) out[c][q] = o[c];
+        if (v.x >= P.box[0] && v.x < P.box[1] && v.y >= P.box[2] && v.y < P.box[3] && v.z >= P.box[4] && v.z < P.box[5]) {
+            acc[0].add(lr);
+            acc[1].add(li);
+            acc[2].add(o[2]);
+        }
+        if constexpr (PHS) {
+            // (the weights are zero outside the trimming box)
+            const T m[3] = {lr, li, o[2]};
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if constexpr (sizeof(T) == 8) {
+                    acc6[c] += m[c] * w1;
+                    acc6[3 + c] += m[c] * w2;
+                } else {
+                    acc6f[c].add_product(m[c], w1);
+                    acc6f[3 + c].add_product(m[c], w2);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        if constexpr (sizeof(T) == 8) sums[c][tid] = acc[c].s;
+        else reinterpret_cast<float2*>(sums[c])[tid] = make_float2(acc[c].s, -acc[c].c);
+    }
+    if constexpr (PHS) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+            if constexpr (sizeof(T) == 8) sums[3 + c][tid] = acc6[c];
+            else reinterpret_cast<float2*>(sums[3 + c])[tid] = make_float2(acc6f[c].s, acc6f[c].l);
+        }
+    }
+    chunk_sums<T, NS>(P, k.b, k.c, sums);
+}
+
+// MacCormack over the list (see mac_kernel, bt_step_mac.cuh): the predictor,
+// then the corrector with pulses and sums
+template <typename T, int STAGE, bool VEL, bool PREC, bool PHS>
+__global__ void __launch_bounds__(PT, list_ctas_per_sm(sizeof(T))) pore_mac_kernel(const __grid_constant__ StepParams<T> P) {
+    constexpr int NS = PHS ? 9 : 3;
+    __shared__ double sums[NS][PT];
+    __shared__ PulsePrep pprep;
+
+    const int tid = threadIdx.x;
+    const int nx = P.nx, ny = P.ny, nz = P.nz, pitch = P.pitch;
+    const long long plane = P.plane;
+    const Chunk k = chunk_of(P.npore, P.pchunks, P.nbatch);
+    const unsigned nbt = P.nbatch > 1 ? (unsigned)P.nbatch : 1u;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const long long step = __ldcg(&P.ctl->fstep[P.side]);
+    if (k.adder) {
+        // the predictor adds the previous step's sums, the corrector steps on
+        if constexpr (STAGE == 0) {
+            if (step > __ldcg(&P.ctl->gen_from))
+                add_partials<T, NS>(P, P.partials_prev, P.part6_prev, k.b, step - 1, sums);
+        } else {
+            if (k.b == 0 && tid == 0) P.ctl->fstep[1 - P.side] = step + 1;
+        }
+        return;
+    }
+    const StepInfo* si = P.steps + (step < P.nsched ? step : P.nsched) * nbt + k.b;
+    const T* in[3] = {P.in[0] + k.b * P.bstride, P.in[1] + k.b * P.bstride, P.in[2] + k.b * P.bstride};
+    T* out[3] = {P.out[0] + k.b * P.bstride, P.out[1] + k.b * P.bstride, P.out[2] + k.b * P.bstride};
+    T gd[3] = {0, 0, 0};
+    if constexpr (PREC) {
+        gd[0] = (T)(si->grad[0] * P.dxd);
+        gd[1] = (T)(si->grad[1] * P.dyd);
+        gd[2] = (T)(si->grad[2] * P.dzd);
+    }
+    const int npulse = STAGE == 1 ? si->pulse_count : 0;
+    const DevPulse* pulses = P.pulses + si->pulse_first;
+    if (npulse) {  // CTA-uniform
+        pulse_prep(pprep, pulses, npulse, tid);
+        __syncthreads();
+    }
+    // FP64, as in voxel_step: n along an axis and a gradient along z leave most
+    // products zero; skipped, unless the result is not finite
+    const bool short_form = sizeof(T) == 8 && P.axis >= 0 && P.diffusion;
+    const bool z_only = gd[0] == (T)0 && gd[1] == (T)0;
+    const int bcs[3] = {P.bc[0], P.bc[1], P.bc[2]};
+    const bool bc_live = (bcs[0] | bcs[1] | bcs[2]) != 0 && (STAGE == 1 || step > 0);
+    Acc<T> acc[3];
+    Acc2 acc6f[PHS ? 6 : 1];
+    double acc6[PHS ? 6 : 1] = {};
+
+    for (uint32_t i = k.first + tid; i < k.last; i += PT) {
+        const uint32_t q = P.pidx[i];
+        const int f = P.pcode[i] & 63;
+        const Cell v = cell_of(q, P.by_pitch, P.by_ny, pitch, ny);
+        bool open[6] = {v.x > 0, v.x < nx - 1, v.y > 0, v.y < ny - 1, v.z > 0, v.z < nz - 1};
+        T p0[3], nb[3][6];
+        load_neighbours<T>(in, q, open, pitch, plane, p0, nb);
+        T og[3] = {0, 0, 0};
+        if constexpr (STAGE == 1) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) og[c] = P.orig[c][k.b * P.bstride + q];
+        }
+        T u[3] = {0, 0, 0};
+        if constexpr (VEL) {
+            const T* vx = P.vx + ((long long)v.z * ny + v.y) * P.vxpitch + v.x;
+            const T* vy = P.vy + ((long long)v.z * (ny + 1) + v.y) * pitch + v.x;
+            u[0] = (T)0.5 * (vx[0] + vx[1]) * P.hx;
+            u[1] = (T)0.5 * (vy[0] + vy[pitch]) * P.hy;
+            u[2] = (T)0.5 * (P.vz[q] + P.vz[q + plane]) * P.hz;
+        }
+        const T dtt1 = P.fdtt ? P.fdtt[q] : P.dtt1[f], dtt2 = P.fdtt ? P.fdtt[P.fstride + q] : P.dtt2[f];
+        T df[6];
+#pragma unroll
+        for (int a = 0; a < 6; ++a) df[a] = P.fw ? P.fw[a * P.fstride + q] : (f & (1 << a)) ? P.dps : P.dpp;
+        T w1 = 0, w2 = 0;
+        if constexpr (PHS && STAGE == 1) {
+            w1 = P.phw[q];
+            w2 = P.phw[P.fstride + q];
+        }
+        if (bc_live) {
+            long long far[6];
+            far_cells(v, nx, ny, nz, pitch, plane, far);
+            face_ghosts<T, SCHEME_REF>(bcs, si, in, far, nb, open);
+        }
+        T bb[3] = {0, 0, 0};
+        if constexpr (PREC) {
+            if (!short_form || !z_only) {
+                bb[0] = P.b * (gd[0] * ((T)v.x + (T)0.5));
+                bb[1] = P.b * (gd[1] * ((T)v.y + (T)0.5));
+            }
+            bb[2] = P.b * (gd[2] * ((T)v.z + (T)0.5));
+        }
+        T o[3];
+        auto update = [&](bool whole) {
+            const T div = whole ? P.an[0] * p0[0] + P.an[1] * p0[1] + P.an[2] * p0[2] : (T)0.0;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const T pa = p0[c];
+                T rel;
+                if (whole) {
+                    const T diva = P.an[c] * div;
+                    rel = dtt1 * (P.peqn[c] - diva) + dtt2 * (diva - pa);
+                } else {
+                    rel = P.axis == c ? dtt1 * (P.peqn[c] - pa) : -(dtt2 * pa);
+                }
+                T a = pa + rel;
+                if constexpr (STAGE == 1) a = og[c] + pa + rel;
+                if constexpr (PREC) {
+                    if (whole || !z_only) {
+                        if (c == 0) a += (T)0.0 - bb[1] * p0[2] + bb[2] * p0[1];
+                        if (c == 1) a += (T)0.0 + bb[0] * p0[2] - bb[2] * p0[0];
+                        if (c == 2) a += (T)0.0 - bb[0] * p0[1] + bb[1] * p0[0];
+                    } else {
+                        if (c == 0) a += bb[2] * p0[1];
+                        if (c == 1) a -= bb[2] * p0[0];
+                    }
+                }
+                // the differences of both terms
+                const T xm = pa - nb[c][0], xp = nb[c][1] - pa, ym = pa - nb[c][2], yp = nb[c][3] - pa;
+                const T zm = pa - nb[c][4], zp = nb[c][5] - pa;
+                if (P.diffusion)
+                    a += P.hxx * (df[1] * xp - df[0] * xm) + P.hyy * (df[3] * yp - df[2] * ym) +
+                         P.hzz * (df[5] * zp - df[4] * zm);
+                if constexpr (VEL) {
+                    // a solid neighbour holds the voxel's own value (zero difference)
+                    if constexpr (STAGE == 0)
+                        a += (T)0.0 - u[0] * ((f & 1) ? pa - pa : xm) - u[1] * ((f & 4) ? pa - pa : ym) -
+                             u[2] * ((f & 16) ? pa - pa : zm);
+                    else
+                        a += (T)0.0 - u[0] * ((f & 2) ? pa - pa : xp) - u[1] * ((f & 8) ? pa - pa : yp) -
+                             u[2] * ((f & 32) ? pa - pa : zp);
+                }
+                o[c] = STAGE == 0 ? a : (T)0.5 * a;
+            }
+        };
+        bool whole = !short_form;
+        if (!whole) {
+            update(false);
+            if constexpr (sizeof(T) == 8) whole = not_finite(o[0]) || not_finite(o[1]) || not_finite(o[2]);
+        }
+        if (whole) {
+            if constexpr (PREC) {
+                bb[0] = P.b * (gd[0] * ((T)v.x + (T)0.5));
+                bb[1] = P.b * (gd[1] * ((T)v.y + (T)0.5));
+            }
+            update(true);
+        }
+        if constexpr (STAGE == 1) {
+            if (npulse)
+                apply_pulses<T>(pprep, pulses, npulse, o[0], o[1], o[2], v.x, v.y, v.z, P.dxd, P.dyd, P.dzd, P.gamma, nx,
+                                ny, nz);
+            if (v.x >= P.box[0] && v.x < P.box[1] && v.y >= P.box[2] && v.y < P.box[3] && v.z >= P.box[4] &&
+                v.z < P.box[5]) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) acc[c].add(o[c]);
+            }
+            if constexpr (PHS) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    if constexpr (sizeof(T) == 8) {
+                        acc6[c] += o[c] * w1;
+                        acc6[3 + c] += o[c] * w2;
+                    } else {
+                        acc6f[c].add_product(o[c], w1);
+                        acc6f[3 + c].add_product(o[c], w2);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) out[c][q] = o[c];
+    }
+    if constexpr (STAGE == 1) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if constexpr (sizeof(T) == 8) sums[c][tid] = acc[c].s;
+            else reinterpret_cast<float2*>(sums[c])[tid] = make_float2(acc[c].s, -acc[c].c);
+        }
+        if constexpr (PHS) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                if constexpr (sizeof(T) == 8) sums[3 + c][tid] = acc6[c];
+                else reinterpret_cast<float2*>(sums[3 + c])[tid] = make_float2(acc6f[c].s, acc6f[c].l);
+            }
+        }
+        chunk_sums<T, NS>(P, k.b, k.c, sums);
+    }
+}
+
+// programmatic dependent launch over the list: the CTAs of a step become
+// resident while the previous one drains
+template <typename T, typename K>
+cudaError_t launch_list_kernel(K kernel, const StepParams<T>& p, size_t smem, cudaStream_t s) {
+    const unsigned nb = p.nbatch > 1 ? (unsigned)p.nbatch : 1u;
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = pdl_config(dim3((p.pchunks + 1) * nb), dim3(PT), (int)smem, s, attr);
+    return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
+// the KSPACE kernel's phase tables need more than the 48 KB a kernel gets by
+// default on grids whose edges add up to thousands
+template <typename T, int SCHEME, bool VEL, bool PREC, bool PHS>
+cudaError_t launch_pore_step(const StepParams<T>& p, cudaStream_t s) {
+    const size_t smem = SCHEME == SCHEME_KSPACE ? 2 * sizeof(T) * ((size_t)p.nx + p.ny + p.nz) : 0;
+    auto kernel = pore_step_kernel<T, SCHEME, VEL, PREC, PHS>;
+    if (smem > 40 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    return launch_list_kernel<T>(kernel, p, smem, s);
+}
+
+template <typename T, bool PHS>
+cudaError_t launch_step_list_impl(const StepParams<T>& p, int scheme, int vel, int prec, cudaStream_t s) {
+    if (scheme == SCHEME_REF) {
+        if (vel && prec) return launch_pore_step<T, SCHEME_REF, true, true, PHS>(p, s);
+        if (vel) return launch_pore_step<T, SCHEME_REF, true, false, PHS>(p, s);
+        if (prec) return launch_pore_step<T, SCHEME_REF, false, true, PHS>(p, s);
+        return launch_pore_step<T, SCHEME_REF, false, false, PHS>(p, s);
+    }
+    // (two-component sums are lab-frame sums: not KSPACE)
+    if (vel) return launch_pore_step<T, SCHEME_KSPACE, true, false, false>(p, s);
+    return launch_pore_step<T, SCHEME_KSPACE, false, false, false>(p, s);
+}
+
+template <typename T, int STAGE, bool PHS>
+cudaError_t launch_pore_mac(const StepParams<T>& p, int vel, int prec, cudaStream_t s) {
+    if (vel && prec) return launch_list_kernel<T>(pore_mac_kernel<T, STAGE, true, true, PHS>, p, 0, s);
+    if (vel) return launch_list_kernel<T>(pore_mac_kernel<T, STAGE, true, false, PHS>, p, 0, s);
+    if (prec) return launch_list_kernel<T>(pore_mac_kernel<T, STAGE, false, true, PHS>, p, 0, s);
+    return launch_list_kernel<T>(pore_mac_kernel<T, STAGE, false, false, PHS>, p, 0, s);
+}
+
+// both stages of a MacCormack step
+template <typename T>
+cudaError_t launch_mac_list_impl(const StepParams<T>& p, T* const pred[3], int vel, int prec, cudaStream_t s) {
+    StepParams<T> a = p, b = p;
+    for (int c = 0; c < 3; ++c) {
+        a.out[c] = pred[c];
+        b.orig[c] = p.in[c];
+        b.in[c] = pred[c];
+    }
+    if (p.phw) {
+        cudaError_t e = launch_pore_mac<T, 0, true>(a, vel, prec, s);
+        return e != cudaSuccess ? e : launch_pore_mac<T, 1, true>(b, vel, prec, s);
+    }
+    cudaError_t e = launch_pore_mac<T, 0, false>(a, vel, prec, s);
+    return e != cudaSuccess ? e : launch_pore_mac<T, 1, false>(b, vel, prec, s);
+}
+
+template <typename T>
+cudaError_t launch_list_finish_impl(const StepParams<T>& p, cudaStream_t s) {
+    const unsigned nb = p.nbatch > 1 ? (unsigned)p.nbatch : 1u;
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = pdl_config(dim3(nb), dim3(PT), 0, s, attr);
+    if (p.phw) return cudaLaunchKernelEx(&cfg, list_finish_kernel<T, 9>, p);
+    return cudaLaunchKernelEx(&cfg, list_finish_kernel<T, 3>, p);
+}
+
+}  // namespace bt

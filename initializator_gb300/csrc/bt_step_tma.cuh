@@ -847,23 +847,6 @@ abort:
     __syncthreads();
 }
 
-// programmatic dependent launch: a kernel overlaps its step-independent
-// prologue with the previous launch's tail (BT_NO_PDL turns it off)
-static inline cudaLaunchConfig_t pdl_config(dim3 grid, dim3 block, int smem, cudaStream_t s,
-                                            cudaLaunchAttribute* attr) {
-    static const bool pdl = std::getenv("BT_NO_PDL") == nullptr;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cfg;
-}
-
 template <int SCHEME, bool VEL, bool PREC, int TWV, bool BCK = false, int PH = PH_ALL, bool PAL = false,
           bool RF = false>
 static cudaError_t launch_tma_t(const StepParams<float>& p, const TmaMaps& m, dim3 grid, bool first, cudaStream_t s) {
