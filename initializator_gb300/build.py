@@ -3,6 +3,8 @@
 Translation units are compiled in parallel with nvcc (one -gencode, no cmake):
 
 * ``bt_step_f32.cu`` — FP32 step kernels (default -fmad=true)
+* ``bt_step_quad*.cu`` — the FP32 fast path over the quad list, with the rate
+  palette and for pulse steps
 * ``bt_step_tma64.cu`` — the FP32 fast path for 64-wide tiles (narrow grids)
 * ``bt_step_tma_pal.cu`` — the FP32 fast path with per-voxel rates (rate palette)
 * ``bt_step_f64.cu`` — FP64 step kernels, -fmad=false so that no
@@ -36,6 +38,9 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I" + os.pat
 
 UNITS = [
     ("bt_step_f32.cu", ARCH + ["--ptxas-options=-v"]),
+    ("bt_step_quad.cu", ARCH),
+    ("bt_step_quad_pal.cu", ARCH),
+    ("bt_step_quad_rf.cu", ARCH),
     ("bt_step_tma64.cu", ARCH),
     ("bt_step_tma_pal.cu", ARCH),
     ("bt_step_tma_rf.cu", ARCH + ["--ptxas-options=-v"]),

@@ -1,10 +1,14 @@
 // Host runtime behind include/bt.h: handles, device memory, the per-step
 // schedule table, kernel selection and the CUDA-graph-replayed step loop.
 //
-// Kernel selection per step: FP32 steps without pulses run the TMA fast path
-// (bt_step_tma.cuh); FP64 steps and steps carrying pulses run the generic
-// fused kernel (bt_step.cuh). Runs of GRAPH_STEPS pulse-free steps are
-// replayed from a captured CUDA graph (the step index lives on the device).
+// Kernel selection per step. FP32 fields take the fast path, over the quad list
+// (bt_step_quad.cuh) or, for dense fields well beyond L2, through the TMA ring
+// (bt_step_tma.cuh); FP64 fields, the MacCormack scheme, per-voxel rates beyond
+// the palette, two-component sums and steps with positional or
+// gradient-dependent pulses take the generic kernels over the pore list
+// (bt_step_pore.cuh), or their dense forms (bt_step.cuh, bt_step_mac.cuh) on
+// grids beyond its index. Runs of GRAPH_STEPS pulse-free steps are replayed from
+// a captured CUDA graph (the step index lives on the device).
 #include <cudaTypedefs.h>
 
 #include <algorithm>
@@ -70,6 +74,8 @@ struct bt_handle {
     cudaEvent_t in_ready = nullptr, inbox_free = nullptr;
     bt::StepInfo* steps_d = nullptr;
     long long nsched = 0;
+    // some step of the schedule has pulses: all fixed-angle, or others
+    bool pulse_fixed = false, pulse_general = false;
     std::vector<bt::StepInfo> steps_h;
     std::vector<double> kpos;     // wave vector at the start of each step (KSPACE): [step][batch][3]
     bt::DevPulse* pulses_d = nullptr;
@@ -125,14 +131,27 @@ struct bt_handle {
     uint8_t* pcode = nullptr;
     int* pbox = nullptr;
     uint32_t npore = 0, pchunks = 1;
+    // the quad list of the FP32 fast path; without it (grids beyond its index,
+    // or bt_set_wait_polls) the fast path is the TMA ring
+    bool quad_ok = false, use_quad = false;
+    uint32_t* qhead = nullptr;
+    uint32_t* qcodes = nullptr;
+    float* qvel = nullptr;
+    uint32_t* qpal = nullptr;
+    uint32_t nquad = 0, qchunks = 0;
+    bt::StepParams<float> pq[2];
     // The list kernels leave solid voxels alone, which hold zero in both field
     // buffers unless the caller put something else there: looked over when a
     // field comes in (solid_flag, pinned: read once the stream is idle) or, after
     // bt_field_device gave the field away, at the next run. dirty: the buffers
-    // whose solid voxels have to be cleared before a list kernel writes them.
+    // whose solid voxels have to be cleared before a list kernel writes them, or
+    // the quad kernels read them (which give pore-solid faces a weight);
+    // not_finite: the dirty buffer holds a NaN or Inf in solid, which has to
+    // reach the sums as it always did, through the generic kernel.
     int* solid_flag = nullptr;
     bool solid_unknown = false;
     bool dirty[2] = {false, false};
+    bool not_finite = false;
     bool touched = false;         // a field was set, given away or advanced
 };
 
@@ -150,6 +169,9 @@ int fail(bt_handle* h, int code, const std::string& msg) {
             return fail(h, (e_ == cudaErrorMemoryAllocation) ? BT_E_NOMEM : BT_E_CUDA,               \
                         std::string(#call) + ": " + cudaGetErrorString(e_));                          \
     } while (0)
+
+bool fast_path_config(const bt_config& c);
+bool build_maps(bt_handle* h);
 
 void drop_graphs(bt_handle* h) {
     for (auto& g : h->graph)
@@ -278,6 +300,14 @@ void fill_params(bt_handle* h, bt::StepParams<T>* p, int zsplit, int zlong = 1 <
     }
 }
 
+// entries of a block of the quad list: about eight quads a thread, the same
+// number of blocks for every CTA
+uint32_t quad_block(const bt_handle* h) {
+    const uint64_t per = ((uint64_t)h->nquad + h->qchunks - 1) / std::max(1u, h->qchunks);
+    const uint64_t m = std::max<uint64_t>(1, (per + 512) / 1024);
+    return (uint32_t)std::max<uint64_t>(32, ((per + m - 1) / m + 31) / 32 * 32);
+}
+
 void refresh_params(bt_handle* h) {
     // list steps keep one partials buffer per input side, as the fast path does
     const size_t lpart = 3 * (size_t)h->pchunks * h->nb;
@@ -294,6 +324,22 @@ void refresh_params(bt_handle* h) {
             h->pf[s].partials_prev = h->partials_d + (1 - s) * lpart;
         }
         fill_params<float>(h, h->pt, h->tzsplit, h->tzlong);
+        fill_params<float>(h, h->pq, 1);
+        const size_t qpart = 3 * (size_t)std::max(1u, h->qchunks) * h->nb;
+        for (int s = 0; s < 2; ++s) {
+            bt::StepParams<float>& Q = h->pq[s];
+            Q.partials = h->partials_d + s * qpart;
+            Q.partials_prev = h->partials_d + (1 - s) * qpart;
+            Q.qhead = h->qhead;
+            Q.qcodes = h->qcodes;
+            Q.qvel = h->qvel;
+            Q.qpal = h->qpal;
+            Q.nquad = h->nquad;
+            Q.pchunks = h->qchunks;
+            Q.qblock = quad_block(h);
+            Q.by_pitch = bt::make_fast_div((uint32_t)h->pitch / 4u);
+            Q.phw = nullptr;
+        }
         // the fast path keeps one partials buffer per input side: a step's
         // partials are read by the next step, which writes the other buffer
         for (int s = 0; s < 2; ++s) {
@@ -392,17 +438,23 @@ int grow_partials(bt_handle* h, size_t need) {
 // one or more entries a thread; grids beyond its 31-bit element index (or with
 // edges whose KSPACE phase tables do not fit shared memory) keep the dense
 // kernels
-int build_pore_list(bt_handle* h) {
+bool list_possible(const bt_handle* h) {
     const bt_config& c = h->cfg;
-    h->use_list = false;
-    if (h->pidx) cudaFree(h->pidx);
-    if (h->pcode) cudaFree(h->pcode);
-    if (h->pbox) cudaFree(h->pbox);
+    return h->comp < ((size_t)1 << 31) &&
+           (c.scheme != BT_SCHEME_KSPACE || 2 * h->esz * ((size_t)c.nx + c.ny + c.nz) <= 160 * 1024);
+}
+
+void free_pore_list(bt_handle* h) {
+    for (void* p : {(void*)h->pidx, (void*)h->pcode, (void*)h->pbox})
+        if (p) cudaFree(p);
     h->pidx = nullptr;
     h->pcode = nullptr;
     h->pbox = nullptr;
-    if (h->comp >= ((size_t)1 << 31)) return BT_OK;
-    if (c.scheme == BT_SCHEME_KSPACE && 2 * h->esz * ((size_t)c.nx + c.ny + c.nz) > 160 * 1024) return BT_OK;
+    h->use_list = false;
+}
+
+int build_pore_list(bt_handle* h) {
+    const bt_config& c = h->cfg;
     const uint32_t nseg = bt::list_segments(c.nx, c.ny, c.nz);
     uint32_t* offs = nullptr;
     CK(h, cudaMalloc(&offs, sizeof(uint32_t) * ((size_t)nseg + 1)));
@@ -433,8 +485,99 @@ int build_pore_list(bt_handle* h) {
         CK(h, cudaMalloc(&h->part6_d, sizeof(double) * 6 * std::max<size_t>(SUMS_BLOCKS, 2 * (size_t)h->pchunks)));
     }
     h->use_list = true;
+    refresh_params(h);
     return BT_OK;
 }
+
+void free_quads(bt_handle* h) {
+    for (void* p : {(void*)h->qhead, (void*)h->qcodes, (void*)h->qvel, (void*)h->qpal})
+        if (p) cudaFree(p);
+    h->qhead = nullptr;
+    h->qcodes = nullptr;
+    h->qvel = nullptr;
+    h->qpal = nullptr;
+    h->qchunks = 0;
+    h->quad_ok = h->use_quad = false;
+}
+
+// CTA slots of the quad kernels on the whole GPU
+long long quad_slots(const bt_handle* h) { return (long long)bt::QUAD_CTAS_PER_SM * h->num_sms; }
+
+// the quad kernels' CTAs per member, between one and one a 128 entries
+int set_quad_chunks(bt_handle* h, long long chunks) {
+    const long long most = std::max<long long>(1, ((long long)h->nquad + bt::LIST_THREADS - 1) / bt::LIST_THREADS);
+    const uint32_t n = (uint32_t)std::max<long long>(1, std::min(most, chunks));
+    if (n == h->qchunks) return BT_OK;  // keep the captured graphs
+    h->qchunks = n;
+    int rc = grow_partials(h, 6 * (size_t)n * h->nb);
+    if (rc) return rc;
+    refresh_params(h);
+    return BT_OK;
+}
+
+long long list_columns(const bt_handle* h) {
+    return (long long)((h->cfg.nx + bt::LT_X - 1) / bt::LT_X) * ((h->cfg.ny + bt::LT_Y - 1) / bt::LT_Y);
+}
+
+// default: one wave of CTAs, every SM the same share of the list
+int default_quad_chunks(bt_handle* h) { return set_quad_chunks(h, (quad_slots(h) + h->nb - 1) / h->nb); }
+
+// The list skips solid, the TMA ring streams every voxel at a higher rate: on
+// fields well beyond L2 the ring wins where nearly every quad holds a pore voxel
+// (measured, us a step with flow, list / ring; q = quads with a pore voxel):
+// 256^3 q .67 104 / 107, q .75 114 / 107, q 1 127 / 108; 320 x 160 x 160 q .75 57 /
+// 61, q .81 61 / 61, q 1 66 / 61; 201 x 149 x 131 q 1 37 / 40; a batch of eight
+// 128^3 fields q 1 115 / 117. Small grids: 64^3 q 1 6 / 16.
+bool ring_is_faster(const bt_handle* h) {
+    const double q = 4.0 * (double)h->nquad / (double)h->nvox;
+    return h->nb == 1 && ((h->nvox >= ((size_t)12 << 20) && q > 0.7) || (h->nvox >= ((size_t)6 << 20) && q > 0.85));
+}
+
+// the FP32 fast path's quad list from the geometry code, with the velocities in
+// list order
+int build_quad_list(bt_handle* h) {
+    const bt_config& c = h->cfg;
+    free_quads(h);
+    if (!fast_path_config(c) || !list_possible(h) || h->comp / 4 >= (size_t)bt::QUAD_INDEX) return BT_OK;
+    if (c.scheme == BT_SCHEME_KSPACE && 8 * ((size_t)c.nx + c.ny + c.nz + 4) > 160 * 1024) return BT_OK;
+    const uint32_t nseg = bt::list_segments(c.nx, c.ny, c.nz);
+    uint32_t* offs = nullptr;
+    CK(h, cudaMalloc(&offs, sizeof(uint32_t) * ((size_t)nseg + 1)));
+    cudaError_t e = bt::list_offsets(h->code, c.nx, c.ny, c.nz, h->cpitch, true, offs, h->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h->nquad, offs + nseg, 4, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e == cudaSuccess && ring_is_faster(h)) {
+        cudaFree(offs);
+        return BT_OK;
+    }
+    const size_t n = std::max<size_t>(1, h->nquad);
+    if (e == cudaSuccess) e = cudaMalloc(&h->qhead, 4 * n);
+    if (e == cudaSuccess) e = cudaMalloc(&h->qcodes, 4 * n);
+    if (e == cudaSuccess)
+        e = bt::fill_quad_list(h->code, c.nx, c.ny, c.nz, h->pitch, h->cpitch, offs, h->qhead, h->qcodes, h->stream);
+    if (e == cudaSuccess && c.velocity == 1) e = cudaMalloc(&h->qvel, sizeof(float) * 12 * n);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    cudaFree(offs);
+    CK(h, e);
+    h->quad_ok = h->use_quad = true;
+    int rc = default_quad_chunks(h);
+    if (rc) return rc;
+    if (c.velocity == 1) {
+        CK(h, bt::quad_velocities(h->pq[0], h->qvel, h->stream));
+        CK(h, cudaStreamSynchronize(h->stream));
+    }
+    return BT_OK;
+}
+
+// the uploaded rate palette's indices in list order
+int quad_rates(bt_handle* h) {
+    if (!h->quad_ok) return BT_OK;
+    if (!h->qpal) CK(h, cudaMalloc(&h->qpal, 4 * std::max<size_t>(1, h->nquad)));
+    CK(h, bt::quad_palette(h->qhead, h->nquad, h->pal_idx, h->pitch, h->cpitch, h->qpal, h->stream));
+    return BT_OK;
+}
+
+int set_tma_default(bt_handle* h);
 
 // the fast path's z-chunking: `chunks` chunks per field in total, spread over
 // the tile columns so that they differ by at most one (at least one chunk per
@@ -478,11 +621,37 @@ int default_tma_split(const bt_handle* h) {
     return (int)std::max<long long>(1, zs);
 }
 
+// default chunking: exactly two waves of CTAs where that is at least four chunks
+// a column (their lengths then differ by a quarter at most), else the even split
+// above (256^3: 608 chunks 106 us a step, 19 even chunks a column 115 us)
+int set_tma_default(bt_handle* h) {
+    const long long tiles = tma_tiles(h), chunks = 4LL * h->num_sms / h->nb;
+    if (!std::getenv("BT_TMA_ZSPLIT") && chunks >= 4 * tiles && 8 * chunks <= tiles * h->cfg.nz)
+        return set_tma_chunks(h, chunks);
+    return set_tma_split(h, default_tma_split(h));
+}
+
 // the FP32 fast path serves this configuration (non-copy faces: KSPACE only)
 bool fast_path_config(const bt_config& c) {
     if (c.precision != BT_F32 || c.scheme == BT_SCHEME_MACCORMACK || std::getenv("BT_NO_TMA")) return false;
     return c.scheme == BT_SCHEME_KSPACE ||
            (c.boundary[0] == BT_BC_COPY && c.boundary[1] == BT_BC_COPY && c.boundary[2] == BT_BC_COPY);
+}
+
+// the TMA ring of the fast path: its dense cell velocities and tensor maps
+int ensure_ring(bt_handle* h) {
+    const bt_config& c = h->cfg;
+    if (!fast_path_config(c) || h->tgrid.y == 0) return BT_OK;
+    if (c.velocity == 1) {
+        if (!h->ucell) {
+            CK(h, cudaMalloc(&h->ucell, sizeof(float) * 3 * h->comp));
+            CK(h, cudaMemsetAsync(h->ucell, 0, sizeof(float) * 3 * h->comp, h->stream));
+        }
+        CK(h, bt::launch_cell_velocity(h->pt[0], h->ucell, (long long)h->comp, h->stream));
+        CK(h, cudaStreamSynchronize(h->stream));
+    }
+    h->use_tma = build_maps(h);
+    return BT_OK;
 }
 
 bool step_has_pulse(const bt_handle* h, long long s) {
@@ -495,6 +664,7 @@ cudaError_t finish_fast(bt_handle* h) {
     if (!h->fast_pending) return cudaSuccess;
     h->fast_pending = false;
     h->launches++;
+    if (h->use_quad) return bt::launch_list_finish<float>(h->pq[h->fast_side], h->stream);
     return bt::launch_tma_finish(h->pt[h->fast_side], h->tgrid, h->stream);
 }
 
@@ -515,29 +685,34 @@ cudaError_t launch_one(bt_handle* h, int side, long long abs_step) {
     // (one rotation; not with the rate palette)
     const bool pulse = step_has_pulse(h, abs_step);
     // (two-component sums are part of the list kernels)
-    const bool fast = c.precision == BT_F32 && c.scheme != BT_SCHEME_MACCORMACK && h->use_tma && !h->fields_d &&
+    bool fast = c.precision == BT_F32 && c.scheme != BT_SCHEME_MACCORMACK && (h->use_quad || h->use_tma) && !h->fields_d &&
                       !(h->use_list && h->weights_d) &&
                       (!pulse || (!h->pal_ok && h->steps_h[abs_step * h->nb].rot_ok));
     cudaError_t e;
+    auto clear = [&](int which) {
+        h->launches++;
+        h->dirty[which] = false;
+        return c.precision == BT_F64 ? bt::solid_clear<double>((double*)h->state_base[which], h->code, c.nx, c.ny, c.nz, h->pitch,
+                                                               h->cpitch, (long long)h->comp, h->nb, h->stream)
+                                     : bt::solid_clear<float>((float*)h->state_base[which], h->code, c.nx, c.ny, c.nz, h->pitch,
+                                                              h->cpitch, (long long)h->comp, h->nb, h->stream);
+    };
+    if (fast && h->use_quad && h->dirty[side]) {
+        if (h->not_finite) fast = false;
+        else if ((e = clear(side)) != cudaSuccess) return e;
+    }
     if (h->dirty[1 - side]) {
-        // the output buffer holds a field with something in its solid voxels;
-        // the dense kernels write them
-        h->dirty[1 - side] = false;
-        if (!fast && h->use_list) {
-            h->launches++;
-            e = c.precision == BT_F64 ? bt::solid_clear<double>((double*)h->state_base[1 - side], h->code, c.nx, c.ny, c.nz,
-                                                                h->pitch, h->cpitch, (long long)h->comp, h->nb, h->stream)
-                                      : bt::solid_clear<float>((float*)h->state_base[1 - side], h->code, c.nx, c.ny, c.nz,
-                                                               h->pitch, h->cpitch, (long long)h->comp, h->nb, h->stream);
-            if (e != cudaSuccess) return e;
-        }
+        // (the dense kernels write the solid voxels themselves)
+        if (!(fast ? h->use_quad : h->use_list)) h->dirty[1 - side] = false;
+        else if ((e = clear(1 - side)) != cudaSuccess) return e;
     }
     if (fast) {
         e = finish_list(h);
         if (e != cudaSuccess) return e;
         // a fast step after a fast step adds its predecessor's partials
         h->launches++;
-        e = bt::launch_step_tma(h->pt[side], h->maps[side], c.scheme, vel, prec, h->pal_ok, pulse, h->tgrid,
+        e = h->use_quad ? bt::launch_step_quad(h->pq[side], c.scheme, vel, prec, h->pal_ok, pulse, h->stream)
+                        : bt::launch_step_tma(h->pt[side], h->maps[side], c.scheme, vel, prec, h->pal_ok, pulse, h->tgrid,
                                 h->ttx, !h->fast_pending, h->stream);
         h->fast_pending = true;
         h->fast_side = side;
@@ -585,9 +760,16 @@ cudaError_t launch_one(bt_handle* h, int side, long long abs_step) {
                                         h->stream);
 }
 
+// some step of this handle may run on the generic kernels
+bool generic_steps(const bt_handle* h) {
+    const bool fast = h->cfg.precision == BT_F32 && h->cfg.scheme != BT_SCHEME_MACCORMACK && (h->use_quad || h->use_tma);
+    if (!fast || h->fields_d || h->weights_d || (h->use_quad && h->dirty[h->cur] && h->not_finite)) return true;
+    return h->pulse_general || (h->pal_ok && h->pulse_fixed);
+}
+
 // every step of this handle is a list step (no fast path, or nothing for it)
 bool lists_only(const bt_handle* h) {
-    return h->use_list && !(h->cfg.precision == BT_F32 && h->cfg.scheme != BT_SCHEME_MACCORMACK && h->use_tma &&
+    return h->use_list && !(h->cfg.precision == BT_F32 && h->cfg.scheme != BT_SCHEME_MACCORMACK && (h->use_quad || h->use_tma) &&
                             !h->fields_d && !h->weights_d);
 }
 
@@ -690,6 +872,9 @@ int build_schedule(bt_handle* h, const bt_pulse* pulses, int npulses, const doub
     CK(h, cudaMalloc(&h->pulses_d, sizeof(bt::DevPulse) * dp.size()));
     CK(h, cudaMemcpy(h->steps_d, st.data(), sizeof(bt::StepInfo) * st.size(), cudaMemcpyHostToDevice));
     CK(h, cudaMemcpy(h->pulses_d, dp.data(), sizeof(bt::DevPulse) * dp.size(), cudaMemcpyHostToDevice));
+    h->pulse_fixed = h->pulse_general = false;
+    for (long long s = 0; s < nsched; ++s)
+        if (st[s * nb].pulse_count > 0) (st[s * nb].rot_ok ? h->pulse_fixed : h->pulse_general) = true;
     h->steps_h.swap(st);
     h->nsched = nsched;
     // the axes along which some step's wave vector (at its start or end) is
@@ -919,7 +1104,10 @@ int get_components(bt_handle* h, double* const* dst, const void* const* src, int
 
 // the stream is idle: what the last look at the current field found
 void take_solid_flag(bt_handle* h) {
-    if (*h->solid_flag) h->dirty[h->cur] = true;
+    if (*h->solid_flag) {
+        h->dirty[h->cur] = true;
+        h->not_finite = *h->solid_flag & 2;
+    }
     *h->solid_flag = 0;
 }
 
@@ -1017,10 +1205,6 @@ int bt_create(const bt_config* cfg, bt_handle** out) {
             if (cudaMalloc(&h->vel[a], h->esz * n3[a]) != cudaSuccess) return bail(BT_E_NOMEM);
             cudaMemset(h->vel[a], 0, h->esz * n3[a]);
         }
-        if (fast_path_config(*cfg)) {
-            if (cudaMalloc(&h->ucell, sizeof(float) * 3 * h->comp) != cudaSuccess) return bail(BT_E_NOMEM);
-            cudaMemset(h->ucell, 0, sizeof(float) * 3 * h->comp);
-        }
     }
     if (cfg->precision == BT_F32) {
         h->nstage = h->nvox <= ((size_t)1 << 26) ? 3 : 2;
@@ -1052,7 +1236,7 @@ int bt_create(const bt_config* cfg, bt_handle** out) {
         // odd widths); BT_TMA_TW = 64 / 128 forces one
         h->ttx = ((cfg->nx + 63) / 64) * 64 < ((cfg->nx + 127) / 128) * 128 ? 64 : 128;
         if (const char* e = std::getenv("BT_TMA_TW")) h->ttx = std::atoi(e) == 64 ? 64 : 128;
-        rc = set_tma_split(h, default_tma_split(h));
+        rc = set_tma_default(h);
         if (rc) return bail(rc);
     }
     *out = h;
@@ -1075,9 +1259,8 @@ int bt_destroy(bt_handle* h) {
     if (h->ctl_d) cudaFree(h->ctl_d);
     if (h->ctl_h) cudaFreeHost(h->ctl_h);
     if (h->solid_flag) cudaFreeHost(h->solid_flag);
-    if (h->pidx) cudaFree(h->pidx);
-    if (h->pcode) cudaFree(h->pcode);
-    if (h->pbox) cudaFree(h->pbox);
+    free_pore_list(h);
+    free_quads(h);
     if (h->staging) pinned_put(h->device, h->staging_bytes, h->staging);
     for (auto& e : h->stage_ev)
         if (e) cudaEventDestroy(e);
@@ -1140,10 +1323,6 @@ int bt_upload_geometry(bt_handle* h, const uint8_t* mask, const double* vx, cons
                                    cudaMemcpyHostToDevice));
             }
         }
-        if (h->ucell) {
-            CK(h, bt::launch_cell_velocity(h->pt[0], h->ucell, (long long)h->comp, h->stream));
-            CK(h, cudaStreamSynchronize(h->stream));
-        }
     }
     // a field from before the new geometry may hold something where there is
     // solid now
@@ -1154,10 +1333,14 @@ int bt_upload_geometry(bt_handle* h, const uint8_t* mask, const double* vx, cons
         h->dirty[1 - h->cur] = false;
         h->solid_unknown = true;
     }
-    int rc = build_pore_list(h);
+    free_pore_list(h);
+    refresh_params(h);
+    int rc = build_quad_list(h);
     if (rc) return rc;
+    if (h->wait_polls != bt::RING_WAIT_POLLS) h->use_quad = false;
+    h->use_tma = false;
+    if (!h->use_quad && (rc = ensure_ring(h))) return rc;
     h->geometry = true;
-    if (fast_path_config(h->cfg) && h->tgrid.y > 0) h->use_tma = build_maps(h);
     refresh_params(h);
     return BT_OK;
 }
@@ -1291,6 +1474,8 @@ int run_begin(bt_handle* h, long long nsteps) {
     CK(h, cudaStreamSynchronize(h->stream));
     take_solid_flag(h);
     h->touched = true;
+    // the generic kernels' list, built when they are first needed
+    if (!h->use_list && list_possible(h) && generic_steps(h) && (rc = build_pore_list(h))) return rc;
     h->ctl_h->step = h->step;
     h->ctl_h->mt_base = h->step;
     h->ctl_h->ticket = 0;
@@ -1371,9 +1556,17 @@ int bt_run_many(bt_handle* const* hs, int n, long long nsteps) {
     if (n > 1) {
         long long vox_all = 0;
         for (int i = 0; i < n; ++i)
-            if (hs[i]->use_tma) vox_all += (long long)hs[i]->nvox * hs[i]->nb;
+            if (hs[i]->use_quad || hs[i]->use_tma) vox_all += (long long)hs[i]->nvox * hs[i]->nb;
         for (int i = 0; i < n && vox_all > 0; ++i) {
             bt_handle* h = hs[i];
+            if (h->use_quad) {
+                const double share = (double)h->nvox / (double)vox_all;
+                const long long ch = std::max(1LL, (long long)std::floor(2.0 * quad_slots(h) * share + 0.5));
+                CK(h, cudaStreamSynchronize(h->stream));
+                int rc = set_quad_chunks(h, ch);
+                if (rc) return rc;
+                continue;
+            }
             if (!h->use_tma) continue;
             const bt_config& c = h->cfg;
             const int tw = h->ttx, th = bt::tile_rows(tw);
@@ -1620,6 +1813,7 @@ int build_palette(bt_handle* h, const double* t1, const double* t2, const double
     CK(h, cudaMemcpy(h->pal_tab, tab.data(), 512 * sizeof(float), cudaMemcpyHostToDevice));
     // the tensor maps gain the palette index
     if (h->use_tma) h->use_tma = build_maps(h);
+    if (int rc = quad_rates(h)) return rc;
     h->pal_ok = true;
     return BT_OK;
 }
@@ -1705,6 +1899,7 @@ int bt_upload_rate_palette(bt_handle* h, const double* t1, const double* t2, int
     CK(h, cudaMemcpy2DAsync(h->pal_idx, h->cpitch, idx, c.nx, c.nx, (size_t)c.ny * c.nz, cudaMemcpyDeviceToDevice,
                             h->stream));
     CK(h, cudaMemcpyAsync(h->pal_tab, tab.data(), 512 * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+    if (int rc = quad_rates(h)) return rc;
     CK(h, cudaStreamSynchronize(h->stream));  // tab is a host temporary
     if (h->use_tma) h->use_tma = build_maps(h);
     h->pal_ok = true;
@@ -1779,29 +1974,37 @@ int bt_set_wait_polls(bt_handle* h, long long polls) {
     if (!h) return BT_E_ARG;
     CK(h, cudaStreamSynchronize(h->stream));
     h->wait_polls = polls < 0 ? bt::RING_WAIT_POLLS : (uint32_t)std::min<long long>(polls, 0xffffffffLL);
+    // only the ring waits: a shortened bound puts the fast path on it
+    h->use_quad = h->quad_ok && h->wait_polls == bt::RING_WAIT_POLLS;
+    if (!h->use_quad && h->geometry && !h->use_tma) {
+        int rc = ensure_ring(h);
+        if (rc) return rc;
+    }
     refresh_params(h);  // the parameters are baked into the captured graphs
     return BT_OK;
 }
 
 int bt_set_tma_split(bt_handle* h, int zsplit) {
     if (!h) return BT_E_ARG;
-    if (h->cfg.precision != BT_F32 || !h->use_tma) return BT_OK;  // no fast path on this handle
+    if (h->cfg.precision != BT_F32 || !(h->use_quad || h->use_tma)) return BT_OK;  // no fast path on this handle
     CK(h, cudaStreamSynchronize(h->stream));
-    return set_tma_split(h, zsplit > 0 ? zsplit : default_tma_split(h));
+    if (h->use_quad) return zsplit > 0 ? set_quad_chunks(h, zsplit * list_columns(h)) : default_quad_chunks(h);
+    return zsplit > 0 ? set_tma_split(h, zsplit) : set_tma_default(h);
 }
 
 int bt_set_tma_chunks(bt_handle* h, int chunks) {
     if (!h) return BT_E_ARG;
-    if (h->cfg.precision != BT_F32 || !h->use_tma) return BT_OK;  // no fast path on this handle
+    if (h->cfg.precision != BT_F32 || !(h->use_quad || h->use_tma)) return BT_OK;  // no fast path on this handle
     CK(h, cudaStreamSynchronize(h->stream));
-    if (chunks <= 0) return set_tma_split(h, default_tma_split(h));
+    if (h->use_quad) return chunks > 0 ? set_quad_chunks(h, chunks) : default_quad_chunks(h);
+    if (chunks <= 0) return set_tma_default(h);
     return set_tma_chunks(h, chunks);
 }
 
 int bt_autotune(bt_handle* h, int trial_steps, int* best_chunks) {
     if (!h || trial_steps <= 0) return fail(h, BT_E_ARG, "bad autotune arguments");
     if (!h->geometry) return fail(h, BT_E_STATE, "bt_upload_geometry first");
-    if (h->cfg.precision != BT_F32 || !h->use_tma) {
+    if (h->cfg.precision != BT_F32 || !(h->use_quad || h->use_tma)) {
         if (best_chunks) *best_chunks = h->gzsplit;
         return BT_OK;
     }
@@ -1827,8 +2030,15 @@ int bt_autotune(bt_handle* h, int trial_steps, int* best_chunks) {
         add((below + 1) * tiles);
     }
     cand.push_back((long long)default_tma_split(h) * tiles);
-    std::sort(cand.begin(), cand.end());
-    cand.erase(std::unique(cand.begin(), cand.end()), cand.end());
+    auto use = [&](long long ch) { return h->use_quad ? set_quad_chunks(h, ch) : set_tma_chunks(h, ch); };
+    auto now = [&]() { return h->use_quad ? (long long)h->qchunks : (long long)(h->tzsplit - 1) * tiles + h->tzlong; };
+    if (h->use_quad) {
+        // the quad list: one to eight waves of CTAs over all members, and chunks
+        // of eight entries a thread
+        cand.clear();
+        for (long long w : {1, 2, 3, 4, 6, 8}) cand.push_back(std::max(1LL, (w * quad_slots(h) + h->nb - 1) / h->nb));
+        cand.push_back((long long)h->nquad / (8 * bt::LIST_THREADS) + 1);
+    }
     // the trial runs advance the field; the caller's field and step are restored
     const long long step0 = h->step;
     const int cur0 = h->cur;
@@ -1840,12 +2050,12 @@ int bt_autotune(bt_handle* h, int trial_steps, int* best_chunks) {
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     float best = 1e30f;
-    long long best_ch = (long long)(h->tzsplit - 1) * tiles + h->tzlong;
+    long long best_ch = now();
     int rc = BT_OK;
     std::sort(cand.begin(), cand.end());
     cand.erase(std::unique(cand.begin(), cand.end()), cand.end());
     for (long long ch : cand) {
-        if ((rc = set_tma_chunks(h, ch))) break;
+        if ((rc = use(ch))) break;
         if ((rc = bt_run_async(h, GRAPH_STEPS))) break;  // warm-up and graph capture
         cudaEventRecord(e0, h->stream);
         if ((rc = bt_run_async(h, trial_steps))) break;
@@ -1867,11 +2077,11 @@ int bt_autotune(bt_handle* h, int trial_steps, int* best_chunks) {
     cudaFree(keep);
     h->solid_unknown = true;
     if (rc) return rc;
-    rc = set_tma_chunks(h, best_ch);
+    rc = use(best_ch);
     if (rc) return rc;
     rc = bt_set_step(h, step0);
     if (rc) return rc;
-    if (best_chunks) *best_chunks = (int)((long long)(h->tzsplit - 1) * tiles + h->tzlong);
+    if (best_chunks) *best_chunks = (int)now();
     return BT_OK;
 }
 

@@ -175,6 +175,15 @@ struct StepParams {
     uint32_t npore;
     uint32_t pchunks;           // chunks of the list per batch member
     FastDiv by_pitch, by_ny;
+    // FP32 fast path over the quad list (bt_list.cuh): heads, codes, gated cell
+    // velocities [3][nquad][4] and palette indices (4 bytes a quad) in list order;
+    // pchunks and by_pitch (then the pitch in quads) are its own
+    const uint32_t* qhead;
+    const uint32_t* qcodes;
+    uint32_t nquad;
+    uint32_t qblock;            // entries of a block; a CTA takes every pchunks-th one
+    const float* qvel;
+    const uint32_t* qpal;
     // two-component sums (OutputX/Y/Z with NCOMP 2): weights [2][nz][ny][pitch],
     // block partials, M(t) x 6; null when switched off
     const T* phw;
@@ -230,6 +239,12 @@ cudaError_t launch_step_tma_palette(const StepParams<float>& p, const TmaMaps& m
 // the fast path's pulse-step instances (bt_step_tma_rf.cu), both tile widths
 cudaError_t launch_step_tma_pulse(const StepParams<float>& p, const TmaMaps& m, int scheme, int vel, int prec,
                                   dim3 grid, int tw, bool first, cudaStream_t s);
+// FP32 fast path over the quad list (bt_step_quad.cu); pal: the rate palette, rf:
+// a step of fixed-angle pulses
+cudaError_t launch_step_quad(const StepParams<float>& p, int scheme, int vel, int prec, bool pal, bool rf,
+                             cudaStream_t s);
+cudaError_t launch_step_quad_pal(const StepParams<float>& p, int scheme, int vel, int prec, cudaStream_t s);
+cudaError_t launch_step_quad_rf(const StepParams<float>& p, int scheme, int vel, int prec, cudaStream_t s);
 cudaError_t launch_tma_finish(const StepParams<float>& p, dim3 grid, cudaStream_t s);
 // upwind cell velocities of the fast path from the face velocities, [axis][z][y][pitch]
 cudaError_t launch_cell_velocity(const StepParams<float>& p, float* u, long long comp, cudaStream_t s);

@@ -3,6 +3,10 @@
 
 namespace bt {
 
+uint32_t list_segments(int nx, int ny, int nz) {
+    return (uint32_t)(((long long)nx + LT_X - 1) / LT_X * ((ny + LT_Y - 1) / LT_Y) * ((nz + LT_Z - 1) / LT_Z) * LT_Z);
+}
+
 namespace {
 
 // geometry code of the four voxels of group (xq, y, z); zero outside
@@ -17,18 +21,36 @@ static_assert(SEG_GROUPS % 32 == 0, "a warp walks a segment");
 
 struct ListGrid {
     int nx, ny, nz, pitch, cpitch, ncx;  // ncx: list columns along x
-    uint32_t nseg;                       // segments: column (x fastest) * nz + z
+    uint32_t ncol;                       // list columns of a slab
+    uint32_t nseg;                       // segments: (slab * ncol + column (x fastest)) * LT_Z + plane of the slab
 };
 
+ListGrid list_grid(int nx, int ny, int nz, int pitch, int cpitch) {
+    const int ncx = (nx + LT_X - 1) / LT_X;
+    const uint32_t ncol = (uint32_t)ncx * ((ny + LT_Y - 1) / LT_Y);
+    return ListGrid{nx, ny, nz, pitch, cpitch, ncx, ncol, list_segments(nx, ny, nz)};
+}
+
 __device__ __forceinline__ void segment_origin(const ListGrid& g, uint32_t s, int& xq0, int& y0, int& z) {
-    z = (int)(s % (uint32_t)g.nz);
-    const uint32_t col = s / (uint32_t)g.nz;
+    const uint32_t sc = s / LT_Z, col = sc % g.ncol;
+    z = (int)(sc / g.ncol * LT_Z + s % LT_Z);
     xq0 = (int)(col % (uint32_t)g.ncx) * LT_Q;
     y0 = (int)(col / (uint32_t)g.ncx) * LT_Y;
 }
 
-// one warp a segment: its pore voxels or its groups that hold one
-__global__ void list_count_kernel(const uint8_t* code, ListGrid g, int groups, uint32_t* counts) {
+// the codes of a quad's pore voxels, 7 bits a voxel
+__device__ __forceinline__ uint32_t pore_codes(uint32_t c) {
+    uint32_t e = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t b = (c >> (8 * i)) & 127u;
+        if (b & CODE_PORE) e |= b << (7 * i);
+    }
+    return e;
+}
+
+// one warp a segment: its pore voxels, or its quads that hold one
+__global__ void list_count_kernel(const uint8_t* code, ListGrid g, int quads, uint32_t* counts) {
     const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
     if (s >= g.nseg) return;
@@ -37,7 +59,7 @@ __global__ void list_count_kernel(const uint8_t* code, ListGrid g, int groups, u
     uint32_t n = 0;
     for (int k = lane; k < SEG_GROUPS; k += 32) {
         const uint32_t c = code4_at(code, xq0 + k % LT_Q, y0 + k / LT_Q, z, g.nx, g.ny, g.nz, g.cpitch) & PORES;
-        n += groups ? (c ? 1u : 0u) : (uint32_t)__popc(c);
+        n += quads ? (c ? 1u : 0u) : (uint32_t)__popc(c);
     }
     n = __reduce_add_sync(0xffffffffu, n);
     if (lane == 0) counts[s] = n;
@@ -119,6 +141,80 @@ __global__ void pore_fill_kernel(const uint8_t* code, ListGrid g, const uint32_t
     }
 }
 
+// one warp a segment: its quads in order
+__global__ void quad_fill_kernel(const uint8_t* code, ListGrid g, const uint32_t* offs, uint32_t* head, uint32_t* codes) {
+    const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x & 31;
+    if (s >= g.nseg) return;
+    int xq0, y0, z;
+    segment_origin(g, s, xq0, y0, z);
+    uint32_t at = offs[s];
+    const int pq = g.pitch / 4;
+    for (int k = lane; k < SEG_GROUPS; k += 32) {
+        const int xl = k % LT_Q, xq = xq0 + xl, y = y0 + k / LT_Q;
+        const uint32_t c = code4_at(code, xq, y, z, g.nx, g.ny, g.nz, g.cpitch);
+        const bool take = (c & PORES) != 0u;
+        const uint32_t vote = __ballot_sync(0xffffffffu, take);
+        if (take) {
+            const uint32_t q = ((uint32_t)z * g.ny + y) * (uint32_t)pq + xq;
+            const uint32_t w = at + __popc(vote & ((1u << lane) - 1u));
+            uint32_t h = q, e = pore_codes(c);
+            if (xl == 0 && xq > 0) h |= QUAD_LEFT;
+            if (xl == LT_Q - 1 && 4 * xq + 4 < g.nx) h |= QUAD_RIGHT;
+            if (xl > 0 && (code4_at(code, xq - 1, y, z, g.nx, g.ny, g.nz, g.cpitch) & PORES)) e |= QUAD_PREV;
+            if (xl < LT_Q - 1 && (code4_at(code, xq + 1, y, z, g.nx, g.ny, g.nz, g.cpitch) & PORES)) e |= QUAD_NEXT;
+            // the sector's other quad (it may be in the next or previous row, or
+            // behind the component)
+            const uint32_t m = q ^ 1u, row = m / pq;
+            if (!(code4_at(code, (int)(m - row * pq), (int)(row % g.ny), (int)(row / g.ny), g.nx, g.ny, g.nz, g.cpitch) &
+                  PORES))
+                e |= QUAD_ALONE;
+            if (xq == 0 || 4 * xq + 4 >= g.nx || y == 0 || y == g.ny - 1 || z == 0 || z == g.nz - 1) e |= QUAD_EDGE;
+            head[w] = h;
+            codes[w] = e;
+        }
+        at += __popc(vote);
+    }
+}
+
+// one thread a quad of the list: its gated cell velocities
+__global__ void quad_velocity_kernel(const StepParams<float> P, float* u) {
+    const float h2[3] = {0.5f * P.hx, 0.5f * P.hy, 0.5f * P.hz};
+    const uint32_t pq = (uint32_t)P.pitch / 4u;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P.nquad; i += gridDim.x * blockDim.x) {
+        const uint32_t q = P.qhead[i] & QUAD_INDEX;
+        const uint32_t row = q / pq;
+        const long long z = row / P.ny, y = row % P.ny;
+        const int x = 4 * (int)(q - row * pq);
+        float v[3][4];
+        for (int j = 0; j < 4; ++j) {
+            const bool inside = x + j < P.nx;
+            const float* vx = P.vx + (long long)row * P.vxpitch + x + j;
+            const float* vy = P.vy + (z * (P.ny + 1) + y) * P.pitch + x + j;
+            const float* vz = P.vz + (long long)row * P.pitch + x + j;
+            for (int a = 0; a < 3; ++a) {
+                const float lo = !inside ? 0.f : a == 0 ? vx[0] : a == 1 ? vy[0] : vz[0];
+                const float hi = !inside ? 0.f : a == 0 ? vx[1] : a == 1 ? vy[P.pitch] : vz[(long long)P.ny * P.pitch];
+                const float w = h2[a] * (lo + hi);
+                v[a][j] = (w < 0.f ? hi != 0.f : lo != 0.f) ? w : 0.f;
+            }
+        }
+        for (int a = 0; a < 3; ++a)
+            reinterpret_cast<float4*>(u)[(size_t)a * P.nquad + i] = make_float4(v[a][0], v[a][1], v[a][2], v[a][3]);
+    }
+}
+
+// one thread a quad of the list: its voxels' palette indices
+__global__ void quad_palette_kernel(const uint32_t* head, uint32_t n, const uint8_t* idx, int pitch, int cpitch,
+                                    uint32_t* out) {
+    const uint32_t pq = (uint32_t)pitch / 4u;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t q = head[i] & QUAD_INDEX;
+        const uint32_t row = q / pq;
+        out[i] = *reinterpret_cast<const uint32_t*>(idx + (size_t)row * cpitch + 4 * (q - row * pq));
+    }
+}
+
 // one CTA a chunk: the bounding box (x0, x1, y0, y1, z0, z1) of its entries
 __global__ void __launch_bounds__(128) chunk_box_kernel(const uint32_t* idx, uint32_t n, uint32_t chunks, FastDiv by_pitch,
                                                         FastDiv by_ny, int pitch, int ny, int* box) {
@@ -150,8 +246,9 @@ __global__ void __launch_bounds__(128) chunk_box_kernel(const uint32_t* idx, uin
     }
 }
 
-// Raises *flag (host memory, read after the stream is synchronised) when a
-// solid voxel of a member's field holds anything but zero; with src, first
+// Sets *flag (host memory, read after the stream is synchronised) when a solid
+// voxel of a member's field holds anything but zero: 1, or 3 when one is not
+// finite; with src, first
 // copies the dense arrays src[c] ([members][nz][ny][nx]) into the field.
 // One thread a group of four voxels.
 template <typename T>
@@ -159,7 +256,7 @@ __global__ void field_in_kernel(T* field, const T* s0, const T* s1, const T* s2,
                                 int nz, int pitch, int cpitch, long long comp, int members, int* flag) {
     const int gq = pitch / 4;
     const long long rows = (long long)ny * nz, n = rows * gq;
-    bool bad = false;
+    int bad = 0;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
         const long long row = q / gq;
         const int x = 4 * (int)(q - row * gq);
@@ -184,11 +281,13 @@ __global__ void field_in_kernel(T* field, const T* s0, const T* s1, const T* s2,
                         if (x + i < nx) v[i] = d[i];
                 }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) bad = bad || (!((c >> (8 * i)) & CODE_PORE) && !(v[i] == (T)0));
+                for (int i = 0; i < 4; ++i)
+                    if (!((c >> (8 * i)) & CODE_PORE) && !(v[i] == (T)0)) bad |= isfinite(v[i]) ? 1 : 3;
             }
         }
     }
-    if (bad) *flag = 1;
+    if (bad == 1) atomicOr(flag, 1);
+    if (bad == 3) atomicOr(flag, 3);
 }
 
 // zero in the solid voxels of a field
@@ -213,22 +312,36 @@ __global__ void solid_clear_kernel(T* field, const uint8_t* code, int nx, int ny
 
 }  // namespace
 
-uint32_t list_segments(int nx, int ny, int nz) {
-    return (uint32_t)(((long long)nx + LT_X - 1) / LT_X * ((ny + LT_Y - 1) / LT_Y) * nz);
-}
-
-cudaError_t list_offsets(const uint8_t* code, int nx, int ny, int nz, int cpitch, bool groups, uint32_t* offs,
+cudaError_t list_offsets(const uint8_t* code, int nx, int ny, int nz, int cpitch, bool quads, uint32_t* offs,
                          cudaStream_t s) {
-    const ListGrid g{nx, ny, nz, 0, cpitch, (nx + LT_X - 1) / LT_X, list_segments(nx, ny, nz)};
-    list_count_kernel<<<(g.nseg + 7) / 8, 256, 0, s>>>(code, g, groups ? 1 : 0, offs);
+    const ListGrid g = list_grid(nx, ny, nz, 0, cpitch);
+    list_count_kernel<<<(g.nseg + 7) / 8, 256, 0, s>>>(code, g, quads ? 1 : 0, offs);
     list_scan_kernel<<<1, 1024, 0, s>>>(offs, g.nseg);
     return cudaGetLastError();
 }
 
 cudaError_t fill_pore_list(const uint8_t* code, int nx, int ny, int nz, int pitch, int cpitch, const uint32_t* offs,
                            uint32_t* idx, uint8_t* pcode, cudaStream_t s) {
-    const ListGrid g{nx, ny, nz, pitch, cpitch, (nx + LT_X - 1) / LT_X, list_segments(nx, ny, nz)};
+    const ListGrid g = list_grid(nx, ny, nz, pitch, cpitch);
     pore_fill_kernel<<<(g.nseg + 7) / 8, 256, 0, s>>>(code, g, offs, idx, pcode);
+    return cudaGetLastError();
+}
+
+cudaError_t fill_quad_list(const uint8_t* code, int nx, int ny, int nz, int pitch, int cpitch, const uint32_t* offs,
+                           uint32_t* head, uint32_t* codes, cudaStream_t s) {
+    const ListGrid g = list_grid(nx, ny, nz, pitch, cpitch);
+    quad_fill_kernel<<<(g.nseg + 7) / 8, 256, 0, s>>>(code, g, offs, head, codes);
+    return cudaGetLastError();
+}
+
+cudaError_t quad_velocities(const StepParams<float>& p, float* u, cudaStream_t s) {
+    quad_velocity_kernel<<<1216, 256, 0, s>>>(p, u);
+    return cudaGetLastError();
+}
+
+cudaError_t quad_palette(const uint32_t* head, uint32_t n, const uint8_t* idx, int pitch, int cpitch, uint32_t* out,
+                         cudaStream_t s) {
+    quad_palette_kernel<<<1216, 256, 0, s>>>(head, n, idx, pitch, cpitch, out);
     return cudaGetLastError();
 }
 

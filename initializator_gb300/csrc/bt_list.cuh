@@ -8,9 +8,11 @@
 // reference never updates them, cpp:3174, 2501-2506) and which the host
 // runtime now keeps (bt_api.cu, solid_check).
 //
-// Order: columns of LT_X x LT_Y voxels, each marching in z, x fastest within a
-// plane, so that the entries one CTA takes in a row are a compact block whose
-// neighbours in y and z come from its own L1.
+// Order: slabs of LT_Z planes; in a slab, columns of LT_X x LT_Y voxels, each
+// marching in z, x fastest within a plane. The entries one CTA takes in a row
+// are a compact block whose neighbours in y and z come from its own L1, and the
+// CTAs that run at the same time cover neighbouring columns, whose shared rows
+// come from L2.
 #pragma once
 #include <algorithm>
 
@@ -20,11 +22,28 @@ namespace bt {
 
 constexpr int LT_X = 64;  // voxels along x of a list column (16 groups of four)
 constexpr int LT_Y = 8;   // rows of a list column
+constexpr int LT_Z = 16;  // planes of a slab
 constexpr int LT_Q = LT_X / 4;
 // generic list kernels: threads of a CTA, and resident CTAs a SM (a launch has
 // as many chunks, one wave: every SM gets the same share of the list)
 constexpr int LIST_THREADS = 128;
 constexpr int list_ctas_per_sm(size_t esz) { return esz == 8 ? 4 : 5; }
+
+// Entry of the quad list, a group of four voxels along x (a quad) that holds a
+// pore voxel. head: the quad's index (elements / 4) within a component, and
+// whether its outer voxels' x neighbours lie in another list column; codes: the
+// voxels' geometry codes, 7 bits each (zero for solid), and flags.
+constexpr uint32_t QUAD_INDEX = (1u << 30) - 1u;
+constexpr uint32_t QUAD_LEFT = 1u << 30, QUAD_RIGHT = 1u << 31;
+constexpr uint32_t QUAD_ALONE = 1u << 28;  // the other quad of its 32-byte sector holds no pore voxel
+constexpr uint32_t QUAD_PREV = 1u << 29;   // the previous entry is the quad at its left
+constexpr uint32_t QUAD_NEXT = 1u << 30;   // the next entry is the quad at its right
+constexpr uint32_t QUAD_EDGE = 1u << 31;   // it touches a face of the domain
+// resident CTAs a SM of the quad kernels: 4 at 128 registers. 3 (168 registers)
+// suits very sparse rocks better (512 x 384 x 256 at 20 %: 150 -> 140 us) and
+// everything else worse (256^3 sphere pack 104 -> 108, 12 uneven samples 145 ->
+// 155 us); 5 spills.
+constexpr int QUAD_CTAS_PER_SM = 4;
 
 // the coordinates of element `idx` of a pitched component
 struct Cell {
@@ -60,15 +79,23 @@ __host__ __device__ inline Cell cell_of(uint32_t idx, const FastDiv& by_pitch, c
 // planes of list columns; offs of list_offsets holds one more
 uint32_t list_segments(int nx, int ny, int nz);
 // offs[segments + 1]: where each segment's entries begin, and how many there are
-// (pore voxels, or groups of four along x that hold one)
-cudaError_t list_offsets(const uint8_t* code, int nx, int ny, int nz, int cpitch, bool groups, uint32_t* offs,
+// (pore voxels, or quads that hold one)
+cudaError_t list_offsets(const uint8_t* code, int nx, int ny, int nz, int cpitch, bool quads, uint32_t* offs,
                          cudaStream_t s);
 cudaError_t fill_pore_list(const uint8_t* code, int nx, int ny, int nz, int pitch, int cpitch, const uint32_t* offs,
                            uint32_t* idx, uint8_t* pcode, cudaStream_t s);
+cudaError_t fill_quad_list(const uint8_t* code, int nx, int ny, int nz, int pitch, int cpitch, const uint32_t* offs,
+                           uint32_t* head, uint32_t* codes, cudaStream_t s);
+// gated cell velocities (see cell_velocity_kernel) of the quads in list order,
+// u[axis][n] float4; palette indices of their voxels, 4 bytes a quad
+cudaError_t quad_velocities(const StepParams<float>& p, float* u, cudaStream_t s);
+cudaError_t quad_palette(const uint32_t* head, uint32_t n, const uint8_t* idx, int pitch, int cpitch, uint32_t* out,
+                         cudaStream_t s);
 // the bounding box of each chunk of a list of element indices
 cudaError_t chunk_boxes(const uint32_t* idx, uint32_t n, uint32_t chunks, const FastDiv& by_pitch, const FastDiv& by_ny,
                         int pitch, int ny, int* box, cudaStream_t s);
-// a field's solid voxels looked over (*flag = 1 where one is not zero), after
+// a field's solid voxels looked over (*flag 1 where one is not zero, 3 where one
+// is not finite), after
 // dense arrays were copied in when src is given
 template <typename T>
 cudaError_t field_in(T* field, const T* const* src, const uint8_t* code, int nx, int ny, int nz, int pitch, int cpitch,

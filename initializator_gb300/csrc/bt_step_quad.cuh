@@ -1,0 +1,500 @@
+// FP32 fast path of the fused step over the quad list: one thread a group of
+// four voxels along x (a quad) that holds a pore voxel.
+//
+// What bounds it: HBM, and the L1 data path and its latency (256^3 sphere pack at
+// 60 % porosity with flow, ncu: DRAM 4.9 TB/s, LSU data pipe 64 %, issue 45 %).
+// The TMA ring streams every voxel and issues ~145 instructions for each, solid or
+// not; the list skips the quads without a pore voxel: a quarter to a third of
+// them in sphere packs, two thirds to three quarters in random-field rocks. Loads
+// are plain 128-bit ones, all of an entry under way before the first is used;
+// list order (bt_list.cuh) makes the entries a CTA takes in a row a compact
+// block, so the rows above, below, in front and behind come from its L1, and the
+// halo values of the quad itself from the neighbouring lanes. No warp waits for
+// another before the sums.
+//
+// Measured, us a step, TMA ring (default chunks) -> list: 64^3 sphere pack 14.8 ->
+// 5.2; 201 x 149 x 131 35 -> 26; 192 x 192 x 128 random field at 25 %, batch of
+// eight, 264 -> 140; 512 x 384 x 256 at 20 % 310 -> 155; 256^3 at 60 % 115 -> 104
+// (ring_is_faster in bt_api.cu has where the ring stays). Tried and slower at 256^3:
+// the next entry's new rows and velocities copied ahead by cp.async (118; it takes
+// the L1 the rows need) or prefetched (123); bricks of two or four planes rolling
+// through registers (122 to 135: fewer loads under way at once); packed FP32 pairs
+// (104: 10 % fewer instructions, no faster); list columns of 32 to 128 voxels by
+// 4 to 16 rows and slabs of 8 to 32 planes (within 4 %).
+//
+// The update is step_tma_kernel's (weights of the six faces, gated cell
+// velocities, face phases of the schedule's axes, the pulse step's rotation,
+// ghosts of domain faces), the protocol of the sums and the step counter the pore
+// list's (bt_step_pore.cuh). A row without an open face towards the quad is not
+// read: the zeros behind the component (index `zero`) stand for it, which is
+// what solid voxels hold.
+#pragma once
+#include "bt_list.cuh"
+#include "bt_step.cuh"
+#include "bt_step_pore.cuh"
+
+namespace bt {
+
+// 128-bit loads with a 64-byte fetch granularity on an L2 miss: the default
+// fetches 128 bytes, half of which a sparse rock does not need (512 x 384 x 256
+// at 20 % porosity: 655 MB read a step at the default, step 162 -> 150 us)
+__device__ __forceinline__ float4 load_row(const float* p) {
+    float4 v;
+    asm volatile("ld.global.L2::64B.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p));
+    return v;
+}
+
+template <int SCHEME, bool VEL, bool PREC, int PH, bool PAL, bool RF>
+__global__ void __launch_bounds__(PT, QUAD_CTAS_PER_SM) quad_step_kernel(const __grid_constant__ StepParams<float> P) {
+    // KSPACE: which axes carry a face phase (see step_tma_kernel)
+    constexpr bool phx = SCHEME == SCHEME_KSPACE && PH == PH_ALL;
+    constexpr bool phz = SCHEME == SCHEME_KSPACE && PH != PH_NONE;
+    constexpr bool ph_axis[3] = {phx, phx, phz};
+    __shared__ double sums[3][PT];
+    // by geometry code: dt/T1, dt/T2, the sum of the open faces' diffusion weights
+    // (zeros for solid)
+    __shared__ float4 s_tab[128];
+    __shared__ float2 s_pal[PAL ? 256 : 1];
+    __shared__ float s_rot[RF ? 12 : 1];
+    extern __shared__ __align__(16) unsigned char phase_raw[];
+    float2* s_ph = reinterpret_cast<float2*>(phase_raw);
+
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int nx = P.nx, ny = P.ny, nz = P.nz;
+    const Chunk k = chunk_of(0u, P.pchunks, P.nbatch);
+    const unsigned nbt = P.nbatch > 1 ? (unsigned)P.nbatch : 1u;
+    const float dm = P.diffusion ? 1.f : 0.f;
+    const float wx = dm * (P.hxx * P.dpp), wy = dm * (P.hyy * P.dpp), wz = dm * (P.hzz * P.dpp);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!k.adder) {
+        // (depends on the launch's parameters only: built while the previous
+        // step drains)
+        for (int q = tid; q < 128; q += PT) {
+            const bool pore = q & CODE_PORE;
+            const float xm = (q & 1) ? 0.f : wx, xp = (q & 2) ? 0.f : wx, ym = (q & 4) ? 0.f : wy,
+                        yp = (q & 8) ? 0.f : wy, zm = (q & 16) ? 0.f : wz, zp = (q & 32) ? 0.f : wz;
+            s_tab[q] = pore ? make_float4(P.dtt1[q & 63], P.dtt2[q & 63], ((xm + xp) + (ym + yp)) + (zm + zp), 0.f)
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if constexpr (PAL) {
+            for (int q = tid; q < 256; q += PT) s_pal[q] = make_float2(P.pal[2 * q], P.pal[2 * q + 1]);
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const long long step = __ldcg(&P.ctl->fstep[P.side]);
+    if (k.adder) {
+        if (k.b == 0 && tid == 0) P.ctl->fstep[1 - P.side] = step + 1;
+        if (step > __ldcg(&P.ctl->gen_from)) add_partials<float, 3>(P, P.partials_prev, nullptr, k.b, step - 1, sums);
+        return;
+    }
+    const StepInfo* si = P.steps + (step < P.nsched ? step : P.nsched) * nbt + k.b;
+    const float* in[3] = {P.in[0] + k.b * P.bstride, P.in[1] + k.b * P.bstride, P.in[2] + k.b * P.bstride};
+    float* out[3] = {P.out[0] + k.b * P.bstride, P.out[1] + k.b * P.bstride, P.out[2] + k.b * P.bstride};
+    if constexpr (RF) {
+        if (tid < 9) s_rot[tid] = si->rotf[tid];
+    }
+    // lab-frame phases of the grid's planes (and columns and rows), FP64-reduced
+    // arguments
+    const int lx = phx ? nx : 0, ly = phx ? ny : 0;
+    if constexpr (phx) {
+        for (int q = tid; q < nx; q += PT) lab_phase<float>(si->knext[0], q, P.dxd, s_ph[q].x, s_ph[q].y);
+        for (int q = tid; q < ny; q += PT) lab_phase<float>(si->knext[1], q, P.dyd, s_ph[lx + q].x, s_ph[lx + q].y);
+    }
+    if constexpr (phz) {
+        for (int q = tid; q < nz; q += PT) lab_phase<float>(si->knext[2], q, P.dzd, s_ph[lx + ly + q].x, s_ph[lx + ly + q].y);
+    }
+    __syncthreads();
+    float gdx = 0.f, gdy = 0.f, gdz = 0.f;
+    if constexpr (PREC && SCHEME == SCHEME_REF) {
+        gdx = (float)(si->grad[0] * P.dxd);
+        gdy = (float)(si->grad[1] * P.dyd);
+        gdz = (float)(si->grad[2] * P.dzd);
+    }
+    float ph[3][2] = {{1.f, 0.f}, {1.f, 0.f}, {1.f, 0.f}};  // exp(+i k d) per axis; the + face uses its conjugate
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        if (ph_axis[a]) {
+            ph[a][0] = si->phasef[a][0];
+            ph[a][1] = si->phasef[a][1];
+        }
+    const uint32_t pq = (uint32_t)P.pitch / 4u, plq = pq * (uint32_t)ny;
+    const uint32_t zero = plq * (uint32_t)nz;  // the zeros behind a component
+    const bool trim = P.box[0] > 0 || P.box[1] < nx || P.box[2] > 0 || P.box[3] < ny || P.box[4] > 0 || P.box[5] < nz;
+    constexpr bool need_cell = phz || (PREC && SCHEME == SCHEME_REF);
+
+    // rows with an open face towards a quad
+    auto open_any = [](uint32_t bits, int f) { return ((bits >> 6) & ~(bits >> f) & 0x00204081u) != 0u; };
+    auto load4 = [](float (&d)[4], const float* p, uint32_t q) {
+        const float4 v = load_row(p + 4ull * q);
+        d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+    };
+
+    Acc<float> acc[3];
+    // This CTA's entries: blocks of P.qblock, every pchunks-th one, so that all
+    // CTAs walk through the list side by side (their shared rows come from L2).
+    // The next entry is read ahead.
+    uint32_t at = k.c * P.qblock, start = at, end = min(P.nquad, at + P.qblock);
+    uint32_t hd = zero, bits0 = 0u;
+    if (at + tid < end) {
+        hd = __ldg(&P.qhead[at + tid]);
+        bits0 = __ldg(&P.qcodes[at + tid]);
+    }
+    while (at < P.nquad) {
+        uint32_t at2 = at + PT, end2 = end;
+        if (at2 >= end) {
+            at2 = start += P.pchunks * P.qblock;
+            end2 = at2 < P.nquad ? min(P.nquad, at2 + P.qblock) : at2;
+        }
+        const uint32_t i = at + tid;
+        const bool live = i < end;
+        const uint32_t quad = hd & QUAD_INDEX, bits = bits0;
+        const bool edge = bits & QUAD_EDGE;
+        // x halo: from the neighbouring lanes where the list goes on with the
+        // neighbouring quad, loaded at the ends of a warp and of a list column
+        const bool from_l = (bits & QUAD_PREV) && lane > 0, from_r = (bits & QUAD_NEXT) && lane < 31 && i + 1 < end;
+        const bool load_l = (hd & QUAD_LEFT) || ((bits & QUAD_PREV) && !from_l);
+        const bool load_r = (hd & QUAD_RIGHT) || ((bits & QUAD_NEXT) && !from_r);
+        hd = zero;
+        bits0 = 0u;
+        if (at2 + tid < end2) {
+            hd = __ldg(&P.qhead[at2 + tid]);
+            bits0 = __ldg(&P.qcodes[at2 + tid]);
+        }
+        int x = 0, y = 0, z = 0;
+        if (need_cell || edge || trim) {
+            const uint32_t row = fast_div(quad, P.by_pitch);  // (by the pitch in quads)
+            z = (int)fast_div(row, P.by_ny);
+            y = (int)row - z * ny;
+            x = 4 * (int)(quad - row * pq);
+        }
+        uint32_t oym = open_any(bits, 2) ? quad - pq : zero, oyp = open_any(bits, 3) ? quad + pq : zero;
+        uint32_t ozm = open_any(bits, 4) ? quad - plq : zero, ozp = open_any(bits, 5) ? quad + plq : zero;
+        if (edge) {
+            if (y == 0) oym = zero;
+            if (y == ny - 1) oyp = zero;
+            if (z == 0) ozm = zero;
+            if (z == nz - 1) ozp = zero;
+        }
+        // every load of the entry is under way before the first is used
+        float hl[3] = {0.f, 0.f, 0.f}, hr[3] = {0.f, 0.f, 0.f};
+        if (load_l && (bits & 0x41u) == 0x40u) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) hl[c] = in[c][4ull * quad - 1];
+        }
+        if (load_r && (bits & (0x42u << 21)) == (0x40u << 21)) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) hr[c] = in[c][4ull * quad + 4];
+        }
+        float cur[3][4], xl[3], xr[3], ym[3][4], yp[3][4], zm[3][4], zp[3][4];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            load4(cur[c], in[c], quad);
+            load4(zp[c], in[c], ozp);
+            load4(ym[c], in[c], oym);
+            load4(yp[c], in[c], oyp);
+            load4(zm[c], in[c], ozm);
+        }
+        float u[3][4] = {};
+        if constexpr (VEL) {
+            // (of entries beyond the block: any velocity, they are zeros throughout)
+            const float* qv = P.qvel + 4ull * min(i, P.nquad - 1u);
+            load4(u[0], qv, 0u);
+            load4(u[1], qv, P.nquad);
+            load4(u[2], qv, 2u * P.nquad);
+        }
+        uint32_t pal4 = 0;
+        if constexpr (PAL) {
+            if (live) pal4 = P.qpal[i];
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float l = __shfl_up_sync(0xffffffffu, cur[c][3], 1), r = __shfl_down_sync(0xffffffffu, cur[c][0], 1);
+            xl[c] = from_l ? l : hl[c];
+            xr[c] = from_r ? r : hr[c];
+        }
+        // (on the x face of the domain the voxel at nx - 1 may be any of the four:
+        // its neighbour then goes into nxt[], else that is the quad's own)
+        float nxt[3][3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) nxt[c][j] = cur[c][j + 1];
+        if (edge) {
+            // ghosts of the domain's faces: copy = the voxel itself, rotated so
+            // that the stencil's face phase brings it back (the first step of a
+            // run from step 0 on every face); zero; periodic = the far edge
+            // cell moved across the period into the k frame
+            auto ghost = [&](float& gr, float& gi, float& gz, float mr, float mi, float mz, int a, bool upper) {
+                // selected, not indexed: a runtime index would put ph in local memory
+                const float c = a == 0 ? ph[0][0] : a == 1 ? ph[1][0] : ph[2][0];
+                const float t = a == 0 ? ph[0][1] : a == 1 ? ph[1][1] : ph[2][1];
+                const float s = upper ? -t : t;
+                gr = (a == 2 ? phz : phx) ? c * mr + s * mi : mr;
+                gi = (a == 2 ? phz : phx) ? c * mi - s * mr : mi;
+                gz = mz;
+            };
+            auto wrap = [&](float& gr, float& gi, float& gz, float mr, float mi, float mz, int a, bool upper) {
+                gr = mr;
+                gi = mi;
+                if constexpr (SCHEME == SCHEME_KSPACE) {
+                    const float c = si->wrapf[a][0], s = upper ? -si->wrapf[a][1] : si->wrapf[a][1];
+                    gr = c * mr - s * mi;
+                    gi = c * mi + s * mr;
+                }
+                gz = mz;
+            };
+            const int kx = step > 0 ? P.bc[0] : BC_COPY, ky = step > 0 ? P.bc[1] : BC_COPY, kz = step > 0 ? P.bc[2] : BC_COPY;
+            const uint32_t rowq = quad - (uint32_t)x / 4u;  // first quad of this row
+            if (x == 0) {
+                if (kx == BC_COPY) ghost(xl[0], xl[1], xl[2], cur[0][0], cur[1][0], cur[2][0], 0, false);
+                if (kx == BC_PERIODIC) {
+                    const size_t o = 4ull * rowq + (nx - 1);
+                    wrap(xl[0], xl[1], xl[2], in[0][o], in[1][o], in[2][o], 0, false);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (x + j == nx - 1) {
+                    float g[3] = {0.f, 0.f, 0.f};
+                    if (kx == BC_COPY) ghost(g[0], g[1], g[2], cur[0][j], cur[1][j], cur[2][j], 0, true);
+                    if (kx == BC_PERIODIC) {
+                        const size_t o = 4ull * rowq;
+                        wrap(g[0], g[1], g[2], in[0][o], in[1][o], in[2][o], 0, true);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) (j < 3 ? nxt[c][j] : xr[c]) = g[c];
+                }
+            auto row_ghosts = [&](float (&g)[3][4], int kind, int a, bool upper, uint32_t far) {
+                if (kind == BC_PERIODIC) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) load4(g[c], in[c], far);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (kind == BC_COPY) ghost(g[0][j], g[1][j], g[2][j], cur[0][j], cur[1][j], cur[2][j], a, upper);
+                    if (kind == BC_PERIODIC) wrap(g[0][j], g[1][j], g[2][j], g[0][j], g[1][j], g[2][j], a, upper);
+                }
+            };
+            if (y == 0) row_ghosts(ym, ky, 1, false, quad + (uint32_t)(ny - 1) * pq);
+            if (y == ny - 1) row_ghosts(yp, ky, 1, true, quad - (uint32_t)(ny - 1) * pq);
+            if (z == 0) row_ghosts(zm, kz, 2, false, quad + (uint32_t)(nz - 1) * plq);
+            if (z == nz - 1) row_ghosts(zp, kz, 2, true, quad - (uint32_t)(nz - 1) * plq);
+        }
+        float er0 = 1.f, ei0 = 0.f;  // exp(-i (k_y y + k_z z)) of this row
+        if constexpr (phx) {
+            const float2 ey = s_ph[lx + (live ? y : 0)], ez = s_ph[lx + ly + (live ? z : 0)];
+            er0 = ey.x * ez.x - ey.y * ez.y;
+            ei0 = ey.x * ez.y + ey.y * ez.x;
+        } else if constexpr (phz) {
+            const float2 ez = s_ph[live ? z : 0];
+            er0 = ez.x;
+            ei0 = ez.y;
+        }
+        float o[3][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t cd = (bits >> (7 * j)) & 127u;
+            const float4 tb = s_tab[cd];
+            // a pore-solid face's neighbour is zero: every face takes the open
+            // faces' weight, and only their sum tells them apart
+            float wxm = wx, wxp = wx, wym = wy, wyp = wy, wzm = wz, wzp = wz;
+            float dtt1 = tb.x, dtt2 = tb.y, wsum = tb.z;
+            if constexpr (PAL) {
+                const float2 r = s_pal[(pal4 >> (8 * j)) & 255u];
+                dtt1 = r.x;
+                dtt2 = r.y;
+            }
+            if constexpr (VEL) {
+                // upwind: +face -min(u,0), -face +max(u,0); their sum is |u|
+                wxp -= fminf(u[0][j], 0.f);
+                wxm += fmaxf(u[0][j], 0.f);
+                wyp -= fminf(u[1][j], 0.f);
+                wym += fmaxf(u[1][j], 0.f);
+                wzp -= fminf(u[2][j], 0.f);
+                wzm += fmaxf(u[2][j], 0.f);
+                wsum = ((wsum + fabsf(u[0][j])) + fabsf(u[1][j])) + fabsf(u[2][j]);
+            }
+            float xm[3], xp[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                xm[c] = j > 0 ? cur[c][j - 1] : xl[c];
+                xp[c] = j < 3 ? nxt[c][j] : xr[c];
+            }
+            const float px0 = cur[0][j], py0 = cur[1][j], pz0 = cur[2][j];
+            float ax, ay, az;
+            // the six faces and the voxel itself, real weights
+            auto faces = [&](int c) {
+                float t = fmaf(wxp, xp[c], wxm * xm[c]);
+                t = fmaf(wyp, yp[c][j], fmaf(wym, ym[c][j], t));
+                t = fmaf(wzp, zp[c][j], fmaf(wzm, zm[c][j], t));
+                return fmaf(-wsum, cur[c][j], t);
+            };
+            if constexpr (SCHEME == SCHEME_REF) {
+                const float div = P.an[0] * px0 + P.an[1] * py0 + P.an[2] * pz0;
+                const float divx = P.an[0] * div, divy = P.an[1] * div, divz = P.an[2] * div;
+                ax = px0 + dtt1 * (P.peqn[0] - divx) + dtt2 * (divx - px0);
+                ay = py0 + dtt1 * (P.peqn[1] - divy) + dtt2 * (divy - py0);
+                az = pz0 + dtt1 * (P.peqn[2] - divz) + dtt2 * (divz - pz0);
+                if constexpr (PREC) {
+                    const float bbxb = P.b * (gdx * ((float)(x + j) + 0.5f));
+                    const float bbyb = P.b * (gdy * ((float)y + 0.5f));
+                    const float bbzb = P.b * (gdz * ((float)z + 0.5f));
+                    ax += bbzb * py0 - bbyb * pz0;
+                    ay += bbxb * pz0 - bbzb * px0;
+                    az += bbyb * px0 - bbxb * py0;
+                }
+                ax += faces(0);
+                ay += faces(1);
+            } else {
+                ax = px0 - dtt2 * px0;
+                ay = py0 - dtt2 * py0;
+                az = pz0 + dtt1 * (P.peqn[2] - pz0);
+                // per axis: w- e^{+i th} m- + w+ e^{-i th} m+
+                //   = cos th (p + q) + i sin th (p - q),  p = w- m-, q = w+ m+
+                // (at th = 0 axis_real's bits: a batch member without a gradient
+                // steps like a single field)
+                auto axis = [&](float wm, float wp, float mr, float mi, float nr, float ni, float c, float s, float& accr,
+                                float& acci) {
+                    const float qr = wp * nr, qi = wp * ni;
+                    accr += fmaf(c, fmaf(wm, mr, qr), -(s * fmaf(wm, mi, -qi)));
+                    acci += fmaf(c, fmaf(wm, mi, qi), s * fmaf(wm, mr, -qr));
+                };
+                auto axis_real = [&](float wm, float wp, float mr, float mi, float nr, float ni, float& accr, float& acci) {
+                    accr += fmaf(wm, mr, wp * nr);
+                    acci += fmaf(wm, mi, wp * ni);
+                };
+                float tr = -(wsum * px0), ti = -(wsum * py0);
+                if constexpr (phx) {
+                    axis(wxm, wxp, xm[0], xm[1], xp[0], xp[1], ph[0][0], ph[0][1], tr, ti);
+                    axis(wym, wyp, ym[0][j], ym[1][j], yp[0][j], yp[1][j], ph[1][0], ph[1][1], tr, ti);
+                } else {
+                    axis_real(wxm, wxp, xm[0], xm[1], xp[0], xp[1], tr, ti);
+                    axis_real(wym, wyp, ym[0][j], ym[1][j], yp[0][j], yp[1][j], tr, ti);
+                }
+                if constexpr (phz) axis(wzm, wzp, zm[0][j], zm[1][j], zp[0][j], zp[1][j], ph[2][0], ph[2][1], tr, ti);
+                else axis_real(wzm, wzp, zm[0][j], zm[1][j], zp[0][j], zp[1][j], tr, ti);
+                ax += tr;
+                ay += ti;
+            }
+            az += faces(2);
+            const bool pore = cd & CODE_PORE;
+            o[0][j] = pore ? ax : 0.f;
+            o[1][j] = pore ? ay : 0.f;
+            o[2][j] = pore ? az : 0.f;
+        }
+        if constexpr (RF) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                // the step's pulses act on the lab-frame value e m, e =
+                // exp(-i k.r); back: conj(e) times it
+                float er = er0, ei = ei0, lr = o[0][j], li = o[1][j];
+                if constexpr (SCHEME == SCHEME_KSPACE) {
+                    if constexpr (phx) {
+                        const float2 ex = s_ph[live ? min(x + j, nx - 1) : 0];
+                        er = ex.x * er0 - ex.y * ei0;
+                        ei = ex.x * ei0 + ex.y * er0;
+                    }
+                    lr = er * o[0][j] - ei * o[1][j];
+                    li = er * o[1][j] + ei * o[0][j];
+                }
+                const float lz = o[2][j];
+                const float nr = s_rot[0] * lr + s_rot[1] * li + s_rot[2] * lz;
+                const float ni = s_rot[3] * lr + s_rot[4] * li + s_rot[5] * lz;
+                o[2][j] = s_rot[6] * lr + s_rot[7] * li + s_rot[8] * lz;
+                if constexpr (SCHEME == SCHEME_KSPACE) {
+                    o[0][j] = er * nr + ei * ni;
+                    o[1][j] = er * ni - ei * nr;
+                } else {
+                    o[0][j] = nr;
+                    o[1][j] = ni;
+                }
+            }
+        }
+        // this quad's sums (solid voxels are zero), in the lab frame
+        float sm[3][4];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sm[c][j] = o[c][j];
+        if (trim) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (!(x + j >= P.box[0] && x + j < P.box[1] && y >= P.box[2] && y < P.box[3] && z >= P.box[4] && z < P.box[5]))
+                    sm[0][j] = sm[1][j] = sm[2][j] = 0.f;
+        }
+        float sx_r = 0.f, sx_i = 0.f, sz_ = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if constexpr (phx) {
+                const float2 ex = s_ph[live ? min(x + j, nx - 1) : 0];
+                sx_r += ex.x * sm[0][j] - ex.y * sm[1][j];
+                sx_i += ex.x * sm[1][j] + ex.y * sm[0][j];
+            } else {
+                sx_r += sm[0][j];
+                sx_i += sm[1][j];
+            }
+            sz_ += sm[2][j];
+        }
+        if constexpr (phz) {
+            acc[0].add(er0 * sx_r - ei0 * sx_i);
+            acc[1].add(er0 * sx_i + ei0 * sx_r);
+        } else {
+            acc[0].add(sx_r);
+            acc[1].add(sx_i);
+        }
+        acc[2].add(sz_);
+        if (live) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                *reinterpret_cast<float4*>(out[c] + 4ull * quad) = make_float4(o[c][0], o[c][1], o[c][2], o[c][3]);
+            if (bits & QUAD_ALONE) {
+                // the other quad of this 32-byte sector holds no pore voxel: its
+                // zeros complete the sector, which then goes to HBM without
+                // being read for the rest of it
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    *reinterpret_cast<float4*>(out[c] + 4ull * (quad ^ 1u)) = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+        at = at2;
+        end = end2;
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) reinterpret_cast<float2*>(sums[c])[tid] = make_float2(acc[c].s, -acc[c].c);
+    chunk_sums<float, 3>(P, k.b, k.c, sums);
+}
+
+template <int SCHEME, bool VEL, bool PREC, int PH, bool PAL, bool RF>
+static cudaError_t launch_quad(const StepParams<float>& p, cudaStream_t s) {
+    const size_t smem = SCHEME == SCHEME_KSPACE && PH != PH_NONE
+                            ? sizeof(float2) * ((PH == PH_ALL ? (size_t)p.nx + p.ny : 0) + p.nz)
+                            : 0;
+    auto kernel = quad_step_kernel<SCHEME, VEL, PREC, PH, PAL, RF>;
+    if (smem > 40 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    return launch_list_kernel<float>(kernel, p, smem, s);
+}
+
+template <bool PAL, bool RF>
+static cudaError_t launch_quad_step(const StepParams<float>& p, int scheme, int vel, int prec, cudaStream_t s) {
+    if (scheme == SCHEME_REF) {
+        if (vel && prec) return launch_quad<SCHEME_REF, true, true, PH_ALL, PAL, RF>(p, s);
+        if (vel) return launch_quad<SCHEME_REF, true, false, PH_ALL, PAL, RF>(p, s);
+        if (prec) return launch_quad<SCHEME_REF, false, true, PH_ALL, PAL, RF>(p, s);
+        return launch_quad<SCHEME_REF, false, false, PH_ALL, PAL, RF>(p, s);
+    }
+    if (p.phase_axes == PH_Z)
+        return vel ? launch_quad<SCHEME_KSPACE, true, false, PH_Z, PAL, RF>(p, s)
+                   : launch_quad<SCHEME_KSPACE, false, false, PH_Z, PAL, RF>(p, s);
+    if (p.phase_axes == PH_NONE)
+        return vel ? launch_quad<SCHEME_KSPACE, true, false, PH_NONE, PAL, RF>(p, s)
+                   : launch_quad<SCHEME_KSPACE, false, false, PH_NONE, PAL, RF>(p, s);
+    return vel ? launch_quad<SCHEME_KSPACE, true, false, PH_ALL, PAL, RF>(p, s)
+               : launch_quad<SCHEME_KSPACE, false, false, PH_ALL, PAL, RF>(p, s);
+}
+
+}  // namespace bt

@@ -1,5 +1,5 @@
-"""The pore-list kernels (generic: one thread a pore voxel) where they can go
-wrong: FP64 against the oracle, bit for bit (array_equal), over field axes that
+"""The list kernels (generic: one thread a pore voxel; FP32 fast path: one a group
+of four along x) where they can go wrong: FP64 against the oracle, bit for bit (array_equal), over field axes that
 take the short relaxation and ones that do not, face velocities at the upwind
 switch's edges (zero, tiny, cancelling pairs), gradients along z alone or along
 every axis; fields that are not finite; fields that are not zero in solid
@@ -138,6 +138,84 @@ def test_list_sizes(shape, porosity, scheme, btlib, oracle_lib):
     tol = 1e-10 if scheme else 0.0  # KSPACE: phase factors differ in rounding
     assert np.abs(got - ref).max() <= tol
     assert np.abs(mt - ref_mt).max() <= max(tol, 1e-12) * max(np.abs(ref_mt).max(), 1.0)
+
+
+@pytest.mark.parametrize("shape,porosity", [((1, 1, 1), 1.0), ((3, 2, 5), 0.6), ((2, 9, 64), 1.0), ((17, 8, 65), 0.3),
+                                            ((5, 7, 63), 0.05), ((33, 17, 130), 0.5), ((4, 4, 8), 0.0)])
+@pytest.mark.parametrize("scheme,axis", [(0, None), (1, None), (1, (0, 0, 1)), (1, (0.3, 0.5, 0.8))])
+@pytest.mark.parametrize("batch,flow,trim", [(1, True, False), (1, False, True), (3, True, True)])
+def test_quad_list_matches_generic(shape, porosity, scheme, axis, batch, flow, trim, btlib, monkeypatch):
+    """The FP32 fast path's quad list against the generic kernel, with a pulse
+    step: the same update in another FP32 order, a few ulps a step (1e-5 over
+    12 steps); any number of chunks gives the same field, M(t) within 1e-6."""
+    import math
+
+    import initializator_gb300 as bt
+    mask, vel, st, kw = _case(shape, 17, porosity=porosity, grad=(0, 0, 0))
+    kw.update(buffer=tuple(min(1, (n - 1) // 2) if trim else 0 for n in reversed(shape)), velocity=int(flow),
+              vector_mult=0)
+    wave = None
+    if scheme == 1:
+        kw.update(gamma=bt.GAMMA_PROTON)
+        if axis is not None:
+            wave = 0.1 * np.ones((12, batch, 1)) * np.linspace(0, 1, batch)[None, :, None] * np.array(axis)
+            wave = wave if batch > 1 else 0.1 * np.ones((12, 1, 1)) * np.array(axis)
+    out = []
+    for env, chunks in (("1", 0), (None, 0), (None, 1), (None, 7)):
+        if env:
+            monkeypatch.setenv("BT_NO_TMA", env)
+        else:
+            monkeypatch.delenv("BT_NO_TMA", raising=False)
+        with bt.Solver(bt.make_config(shape, precision=bt.BT_F32, scheme=scheme, batch=batch, **kw)) as s:
+            s.upload_geometry(mask, vel if flow else None)
+            s.set_schedule([(5, 2, math.pi, (1.0, 0.0, 0.0))], grad_wave=wave)
+            s.set_chunks(chunks)
+            s.set_state(np.stack([st] * batch))
+            mt = s.run(12)
+            out.append((s.get_state(), mt))
+    top = max(np.abs(out[0][1]).max(), 1e-3 * mask.size)
+    assert np.abs(out[1][0] - out[0][0]).max() <= 1e-5
+    assert np.abs(out[1][1] - out[0][1]).max() <= 1e-5 * top
+    for st2, mt2 in out[2:]:
+        assert np.array_equal(st2, out[1][0])
+        assert np.abs(mt2 - out[1][1]).max() <= 1e-6 * top
+
+
+@pytest.mark.parametrize("flow", [False, True])
+def test_dense_large_grid_matches_generic(flow, btlib, monkeypatch):
+    """A field beyond L2 whose quads nearly all hold a pore voxel takes the TMA
+    ring; a shortened wait bound that no wait reaches gives the same bits."""
+    import torch
+
+    import initializator_gb300 as bt
+    shape = (192, 256, 260)
+    rng = np.random.default_rng(3)
+    mask = np.ones(shape, np.uint8)
+    mask[rng.uniform(size=shape) < 0.02] = 0
+    nz, ny, nx = shape
+    vel = None
+    if flow:
+        vel = [rng.uniform(-1e-3, 1e-3, s) for s in ((nz, ny, nx + 1), (nz, ny + 1, nx), (nz + 1, ny, nx))]
+    kw = dict(dx=1e-6, dt=3e-5, d_pore=2.3e-9, t1=0.1, t2=0.05, rho1=1e-5, rho2=1e-5, p_eq=1.0, velocity=int(flow),
+              gamma=bt.GAMMA_PROTON)
+    m = torch.rand(shape, device="cuda") * torch.from_numpy(mask).cuda()
+    out = []
+    for env, polls in (("1", -1), (None, -1), (None, 1 << 19)):
+        if env:
+            monkeypatch.setenv("BT_NO_TMA", env)
+        else:
+            monkeypatch.delenv("BT_NO_TMA", raising=False)
+        with bt.Solver(bt.make_config(shape, precision=bt.BT_F32, scheme=1, **kw)) as s:
+            s.upload_geometry(mask, vel)
+            s.set_wait_polls(polls)
+            s.set_schedule([], grad_wave=np.full((4, 3), 0.05) * (0, 0, 1))
+            s.set_state_device([m, 0.5 * m, m])
+            mt = s.run(4)
+            out.append(([v.clone() for v in s.field_views()], mt))
+    for a, b in zip(out[1][0], out[0][0]):
+        assert float((a - b).abs().max()) <= 1e-5
+    assert np.abs(out[1][1] - out[0][1]).max() <= 1e-5 * np.abs(out[0][1]).max()
+    assert all(torch.equal(a, b) for a, b in zip(out[1][0], out[2][0])) and np.array_equal(out[1][1], out[2][1])
 
 
 def test_geometry_uploaded_again(btlib):
