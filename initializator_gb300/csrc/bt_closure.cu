@@ -9,45 +9,56 @@
 //   * activations are channels-last BF16 in a zero-padded grid, flattened:
 //     row q = voxel of [sample][z+1][y+1][x+1], 16 channels = 32 bytes a row,
 //     with margin rows before and after so every shifted read stays inside;
-//   * a CTA computes 128 consecutive rows (M = 128) x 16 output channels
-//     (N = 16); for each of the 27 taps the A tile is the 128 rows shifted by
-//     the tap's flat offset — one contiguous block, fetched by TMA straight
-//     into the canonical no-swizzle K-major layout (two 2 KB blocks of 8x16-byte
-//     core matrices, one per 8-channel half), K = 16 per MMA;
-//   * the weights of all 27 taps (prepacked on the host in the same canonical
-//     layout, 512 bytes a tap) arrive with one bulk copy;
+//   * a tile is 128 consecutive rows (M = 128) x 16 output channels (N = 16);
+//     for each of the 27 taps its A operand is the 128 rows shifted by the tap's
+//     flat offset, a piece of a window of rows copied into the canonical
+//     no-swizzle K-major layout (8x16-byte core matrices, one plane of them per
+//     8-channel half), K = 16 per MMA;
+//   * the weights of all 27 taps (prepacked in the same canonical layout, 512
+//     bytes a tap) stay in shared memory;
 //   * one thread issues the 27 tcgen05.mma (kind::f16, BF16 x BF16 -> FP32 in
-//     TMEM, 128 lanes x 16 columns), commits to an mbarrier, and the four
-//     warps read their 32 TMEM lanes back (tcgen05.ld 32x32b.x16) for the
-//     epilogue: bias, GELU (or GELU' for the data gradient), store;
+//     TMEM, 128 lanes x 16 columns), commits to mbarriers, and four warps read
+//     their 32 TMEM lanes back (tcgen05.ld 32x32b.x16) for the epilogue: bias,
+//     GELU (or GELU' for the data gradient), store;
 //   * rows that fall on the zero halo are written as zero, so the output is
 //     again a valid padded input for the next layer.
 // The data gradient is the same kernel with the taps reversed and the channel
-// roles swapped (prepacked "dgrad" weights). The weight gradient is a CUDA-core
-// reduction (weight_grad_kernel) with a fixed-order second stage.
+// roles swapped (prepacked "dgrad" weights). The weight gradient is a contraction
+// over the rows (weight_grad_kernel) with a fixed-order second stage.
 // Every mbarrier wait is bounded; a CTA that gives up records status, waits
 // (bounded) for its copies and MMAs, frees its TMEM and returns.
-#include <cuda.h>
 #include <cuda_bf16.h>
-#include <cudaTypedefs.h>
+#include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
 
 #include "../../include/bt.h"
+#include "bt_list.cuh"
 
 namespace {
 
 constexpr int ROWS = 128;        // M: rows (voxels) per CTA
 constexpr int CH = 16;           // channels in and out
 constexpr int TAPS = 27;
-constexpr int A_TAP_BYTES = ROWS * CH * 2;       // 4096
 constexpr int B_TAP_BYTES = CH * CH * 2;         // 512
-constexpr int OFF_A = 0;
-constexpr int OFF_B = TAPS * A_TAP_BYTES;        // 110592
-constexpr int OFF_BAR = OFF_B + TAPS * B_TAP_BYTES;  // 124416
-constexpr int CONV_SMEM = OFF_BAR + 64 + 1024;   // + alignment slack
+// The rows a tile of 128 reads, per half of 8 channels (16 bytes a row): for each
+// dz one window with every (dy, dx), or, where rows are long (xp > 130), for each
+// (dz, dy) one of 130 rows with every dx
+constexpr int WIN_ROWS = ROWS + 2;
+constexpr int A_ROWS = 9 * WIN_ROWS;             // rows of all windows, at most
+constexpr int CONV_STAGES = 8;                   // stages, at most (as many as fit)
+constexpr int CONV_ACC = 8;                      // accumulators of 16 TMEM columns
+constexpr int CONV_SETS = 4;                     // sets of four warps finishing tiles
+constexpr int CONV_MMA_WARP = CONV_STAGES + 4 * CONV_SETS;
+constexpr int CONV_THREADS = 32 * (CONV_MMA_WARP + 1);
+constexpr int OFF_BAR = TAPS * B_TAP_BYTES;      // after the weights
+constexpr int OFF_STAGES = OFF_BAR + 384;
+constexpr int CONV_SMEM = 227 * 1024;
+constexpr int CONV_ROOM = CONV_SMEM - 128 - OFF_STAGES;  // (alignment slack)
+static_assert(OFF_BAR % 128 == 0 && CONV_ROOM >= 4 * (A_ROWS * 32 + 256), "shared memory");
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
 
 __device__ __forceinline__ uint32_t sa(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -56,8 +67,8 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sa(bar)), "r"(count) : "memory");
 }
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sa(bar)), "r"(bytes) : "memory");
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sa(bar)) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
@@ -75,18 +86,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            sa(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(sa(bar))
-        : "memory");
-}
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     sa(dst)),
-                 "l"(src), "r"(bytes), "r"(sa(bar))
-                 : "memory");
+// asynchronous 16-byte copy into shared memory
+__device__ __forceinline__ void copy16(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(sa(dst)), "l"(src) : "memory");
 }
 
 // tcgen05 ------------------------------------------------------------------
@@ -206,7 +208,14 @@ struct ConvParams {
     long long rows;          // padded voxels of the batch (valid rows start at the base row)
     long long base_row;      // margin rows before row 0 in the tensor map / allocations
     int xp, yp, zp;          // padded grid (x+2, y+2, z+2)
-    int taps_off[TAPS];      // flat row offset of each tap
+    int nwin, win_rows;      // windows (3 or 9) and their rows
+    int win_off[9];          // row offset of each window's first row from the tile's
+    int tap_row[TAPS];       // row (over all windows) at which each tap's tile begins
+    int stages, half;        // stages, and bytes of a stage's half
+    const __nv_bfloat16* x;  // padded rows, margin included
+    long long total_rows;
+    bt::FastDiv by_xp, by_plane, by_sample;  // rows < 2^31
+    int vec;                 // pre / outf on 16-byte boundaries
     const unsigned char* wpack;  // 27 x 512 bytes canonical BF16 weights
     const float* bias;       // 16 (forward) or null
     int mode;                // 0: out = GELU(acc + bias) bf16 padded, pre = acc + bias (fp32)
@@ -219,129 +228,386 @@ struct ConvParams {
     int* status;
 };
 
-__global__ void __launch_bounds__(128, 1) conv3d_kernel(const __grid_constant__ ConvParams P,
-                                                        const __grid_constant__ CUtensorMap xmap) {
-    extern __shared__ __align__(1024) unsigned char raw[];
-    unsigned char* sm = raw + ((1024u - (sa(raw) & 1023u)) & 1023u);
-    uint64_t* bar_full = reinterpret_cast<uint64_t*>(sm + OFF_BAR);
-    uint64_t* bar_mma = reinterpret_cast<uint64_t*>(sm + OFF_BAR + 8);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + OFF_BAR + 16);
-    int* s_ok = reinterpret_cast<int*>(sm + OFF_BAR + 24);
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const long long q0 = (long long)blockIdx.x * ROWS;
+// 16 floats of row q of an array of FP32 rows
+__device__ __forceinline__ void row_store(float* p, long long q, const float (&v)[16], int vec) {
+    if (vec) {
+        float4* d = reinterpret_cast<float4*>(p + q * 16);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) d[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+    } else {
+#pragma unroll
+        for (int c = 0; c < 16; ++c) p[q * 16 + c] = v[c];
+    }
+}
+__device__ __forceinline__ void row_load(const float* p, long long q, float (&v)[16], int vec) {
+    if (vec) {
+        const float4* s = reinterpret_cast<const float4*>(p + q * 16);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float4 f = s[c];
+            v[4 * c] = f.x; v[4 * c + 1] = f.y; v[4 * c + 2] = f.z; v[4 * c + 3] = f.w;
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 16; ++c) v[c] = p[q * 16 + c];
+    }
+}
+
+// What bounds it: an MMA with M = 128 and K = 16 takes ~80 cycles here whether N
+// is 16 or 48 (its 4 KB of A), 27 times a tile of 128 rows: 22 us for 8 x 34^3
+// rows with nothing else. So everything else runs beside that. One persistent CTA
+// a SM walks its tiles: a warp a stage copies, one thread issues MMAs, CONV_SETS
+// times four warps finish tiles from CONV_ACC accumulators in TMEM; the weights
+// stay. The taps of a window are the same rows shifted, 16 bytes a row in the
+// no-swizzle layout, which is the unit of a descriptor's start address, so three
+// windows (nine where rows are long) replace 27 shifted tiles, by 16-byte
+// cp.async, as TMA takes 16-byte rows one at a time; each warp waits and fences
+// for its own stage alone. Nine MMAs with N = 48, three taps each, and sums shifted
+// as they are read took 22 us, but add the taps in another order, which BF16
+// between the layers makes visible. A CTA a tile, with 27 tiles by TMA before:
+// 146 us for 8 x 34^3 rows, forward with pre-activation; now 30 us, and 173 us for
+// 130^3 rows.
+__global__ void __launch_bounds__(CONV_THREADS) conv3d_kernel(const __grid_constant__ ConvParams P) {
+    extern __shared__ __align__(128) unsigned char raw[];
+    unsigned char* sm = raw + ((128u - (sa(raw) & 127u)) & 127u);
+    uint64_t* full = reinterpret_cast<uint64_t*>(sm + OFF_BAR);      // a stage's rows are there
+    uint64_t* empty = full + CONV_STAGES;                            // its MMAs are done
+    uint64_t* acc_full = empty + CONV_STAGES;                        // an accumulator is complete
+    uint64_t* acc_empty = acc_full + CONV_ACC;                       // it has been read
+    uint64_t* done = acc_empty + CONV_ACC;                           // every MMA is done
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
+    volatile int* s_ok = reinterpret_cast<int*>(tslot + 1);
+    static_assert((2 * CONV_STAGES + 2 * CONV_ACC + 1) * 8 + 8 <= 384, "barriers");
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const long long ntiles = (P.rows + ROWS - 1) / ROWS;
+    const long long t0 = ntiles * blockIdx.x / gridDim.x, t1 = ntiles * (blockIdx.x + 1) / gridDim.x;
+    const int n = (int)(t1 - t0);
 
     if (tid == 0) {
-        mbar_init(bar_full, 1);
-        mbar_init(bar_mma, 1);
+        for (int i = 0; i < CONV_STAGES; ++i) {
+            mbar_init(&full[i], 32);
+            mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < CONV_ACC; ++i) {
+            mbar_init(&acc_full[i], 1);
+            mbar_init(&acc_empty[i], 128);
+        }
+        mbar_init(done, 1);
         fence_mbar_init();
         *s_ok = 1;
     }
-    if (warp == 0) tmem_alloc(tslot, 32);
+    for (int c = tid; c < TAPS * B_TAP_BYTES / 16; c += CONV_THREADS)
+        reinterpret_cast<uint4*>(sm)[c] = reinterpret_cast<const uint4*>(P.wpack)[c];
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (warp == 0) tmem_alloc(tslot, 16 * CONV_ACC);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
 
-    if (tid == 0) {
-        mbar_expect_tx(bar_full, TAPS * A_TAP_BYTES + TAPS * B_TAP_BYTES);
-        for (int t = 0; t < TAPS; ++t) {
-            const int row = (int)(P.base_row + q0 + P.taps_off[t]);
-            tma_load_2d(sm + OFF_A + t * A_TAP_BYTES, &xmap, bar_full, 0, row);
-            tma_load_2d(sm + OFF_A + t * A_TAP_BYTES + 2048, &xmap, bar_full, 8, row);
+    if (warp < CONV_STAGES) {
+        // copies: this warp's stage, again and again, once the MMAs have read it
+        if (warp < P.stages) {
+            unsigned char* st = sm + OFF_STAGES + warp * 2 * P.half + (lane & 1) * P.half;
+            uint32_t parity = 1u;
+            for (int i = warp; i < n; i += P.stages, parity ^= 1u) {
+                if (!mbar_wait(&empty[warp], parity)) {  // (at once the first time)
+                    *s_ok = 0;
+                    break;
+                }
+                const long long q0 = P.base_row + (t0 + i) * ROWS;
+                for (int w = 0; w < P.nwin; ++w) {
+                    // rows beyond the allocation (a last tile's) belong to no
+                    // result: any row
+                    const long long r0 = q0 + P.win_off[w];
+#pragma unroll 8
+                    for (int r = lane >> 1; r < P.win_rows; r += 16)
+                        copy16(st + (w * P.win_rows + r) * 16, P.x + min(r0 + r, P.total_rows - 1) * 16 + (lane & 1) * 8);
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                mbar_arrive(&full[warp]);
+            }
         }
-        bulk_load(sm + OFF_B, P.wpack, TAPS * B_TAP_BYTES, bar_full);
-        if (!mbar_wait(bar_full, 0)) {
-            *s_ok = 0;
-        } else {
+    } else if (warp == CONV_MMA_WARP) {
+        if (lane == 0) {
+            bool ok = true;
+            const uint64_t bd = smem_desc(sa(sm), 256, 128);
+            int s = 0;
+            uint32_t parity = 0;
+            for (int i = 0; i < n; ++i) {
+                const int a = i % CONV_ACC;
+                ok = mbar_wait(&full[s], parity) && mbar_wait(&acc_empty[a], ((uint32_t)(i / CONV_ACC) & 1u) ^ 1u);
+                if (!ok) break;
+                tc_fence_after();
+                // (a row is one unit of a descriptor's address)
+                const uint64_t ad = smem_desc(sa(sm + OFF_STAGES + s * 2 * P.half), P.half, 128);
+#pragma unroll
+                for (int t = 0; t < TAPS; ++t)
+                    umma_f16(tmem + 16 * a, ad + P.tap_row[t], bd + t * (B_TAP_BYTES / 16), IDESC_BF16_M128_N16, t > 0);
+                umma_commit(&empty[s]);
+                umma_commit(&acc_full[a]);
+                if (++s == P.stages) {
+                    s = 0;
+                    parity ^= 1u;
+                }
+            }
+            // (also when a wait gave up: nothing is in flight when the TMEM goes)
+            umma_commit(done);
+            if (!mbar_wait(done, 0) || !ok) *s_ok = 0;
+        }
+    } else {
+        const int set = (warp - CONV_STAGES) >> 2, quarter = warp & 3;
+        for (int i = set; i < n; i += CONV_SETS) {
+            const int a = i % CONV_ACC;
+            const long long q = (t0 + i) * ROWS + 32 * quarter + lane;
+            // (the data gradient's pre-activations: under way before the wait)
+            float pre[16];
+            if (P.mode == 2 && q < P.rows) row_load(P.pre, q, pre, P.vec);
+            if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[a], (uint32_t)(i / CONV_ACC) & 1u))) {
+                *s_ok = 0;
+                break;
+            }
             tc_fence_after();
-            for (int t = 0; t < TAPS; ++t)
-                umma_f16(tmem, smem_desc(sa(sm + OFF_A + t * A_TAP_BYTES), 2048, 128),
-                         smem_desc(sa(sm + OFF_B + t * B_TAP_BYTES), 256, 128), IDESC_BF16_M128_N16, t > 0);
-            umma_commit(bar_mma);
-            if (!mbar_wait(bar_mma, 0)) *s_ok = 0;
-        }
-    }
-    __syncthreads();
-    if (!*s_ok) {
-        // a bounded wait gave up: record it, let the copies and MMAs in flight
-        // land (bounded), free the TMEM and leave
-        if (tid == 0) {
-            atomicOr(P.status, 8);
-            for (uint32_t i = 0; i < WAIT_LIMIT; ++i)
-                if (mbar_try_wait(bar_full, 0)) break;
-            for (uint32_t i = 0; i < WAIT_LIMIT; ++i)
-                if (mbar_try_wait(bar_mma, 0)) break;
-        }
-        tc_fence_before();
-        __syncthreads();
-        if (warp == 0) tmem_dealloc(tmem, 32);
-        return;
-    }
-    tc_fence_after();
-    float v[16];
-    tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16), v);
-    const long long q = q0 + tid;
-    if (q < P.rows) {
-        // padded coordinates of row q
-        const long long plane = (long long)P.xp * P.yp;
-        const long long r = q % (plane * P.zp);
-        const int z = (int)(r / plane), y = (int)((r / P.xp) % P.yp), x = (int)(r % P.xp);
-        const bool interior = x >= 1 && x <= P.xp - 2 && y >= 1 && y <= P.yp - 2 && z >= 1 && z <= P.zp - 2;
-        if (P.mode == 0 || P.mode == 2) {
+            float v[16];
+            tmem_ld16(tmem + 16 * a + ((uint32_t)(32 * quarter) << 16), v);
+            tc_fence_before();
+            mbar_arrive(&acc_empty[a]);
+            if (q >= P.rows) continue;
+            // padded coordinates of row q
+            uint32_t x, y, z;
+            if (P.rows < (1LL << 31)) {
+                const uint32_t k = (uint32_t)q, smp = bt::fast_div(k, P.by_sample);
+                const uint32_t in = k - smp * (uint32_t)(P.xp * P.yp * P.zp);
+                z = bt::fast_div(in, P.by_plane);
+                const uint32_t p = in - z * (uint32_t)(P.xp * P.yp);
+                y = bt::fast_div(p, P.by_xp);
+                x = p - y * (uint32_t)P.xp;
+            } else {
+                const long long plane = (long long)P.xp * P.yp, in = q % (plane * P.zp);
+                z = (uint32_t)(in / plane);
+                y = (uint32_t)((in / P.xp) % P.yp);
+                x = (uint32_t)(in % P.xp);
+            }
+            const bool interior = x - 1u < (uint32_t)(P.xp - 2) && y - 1u < (uint32_t)(P.yp - 2) && z - 1u < (uint32_t)(P.zp - 2);
+            const float* bias = P.bias;
+            if (P.mode <= 1)
+#pragma unroll
+                for (int c = 0; c < 16; ++c) v[c] += bias[c];
+            if (P.mode == 1 || P.mode == 3) {
+#pragma unroll
+                for (int c = 0; c < 16; ++c) v[c] = interior ? v[c] : 0.f;
+                row_store(P.outf, q, v, P.vec);
+                continue;
+            }
             __align__(16) __nv_bfloat16 o[16];
             if (P.mode == 0) {
 #pragma unroll
                 for (int c = 0; c < 16; ++c) {
-                    const float pre = v[c] + P.bias[c];
-                    if (P.pre) P.pre[q * 16 + c] = interior ? pre : 0.f;
-                    o[c] = __float2bfloat16(interior ? gelu(pre) : 0.f);
+                    v[c] = interior ? v[c] : 0.f;
+                    o[c] = __float2bfloat16(gelu(v[c]));  // gelu(0) = 0
                 }
+                if (P.pre) row_store(P.pre, q, v, P.vec);
             } else {
 #pragma unroll
-                for (int c = 0; c < 16; ++c)
-                    o[c] = __float2bfloat16(interior ? v[c] * gelu_grad(P.pre[q * 16 + c]) : 0.f);
+                for (int c = 0; c < 16; ++c) o[c] = __float2bfloat16(interior ? v[c] * gelu_grad(pre[c]) : 0.f);
             }
             uint4* dst = reinterpret_cast<uint4*>(P.out + (P.base_row + q) * 16);
             dst[0] = reinterpret_cast<const uint4*>(o)[0];
             dst[1] = reinterpret_cast<const uint4*>(o)[1];
-        } else {
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && !*s_ok) atomicOr(P.status, 8);  // a bounded wait gave up
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem, 16 * CONV_ACC);
+}
+
+// ---- weight gradient ----
+// dW[t][ci][co] = sum over rows q of x[q + off_t][ci] dz[q][co] (db[co] as t = 27)
+// is a contraction over hundreds of thousands of rows with 432 x 16 results. On
+// the tensor cores, with the rows as K: both operands have their channels
+// contiguous, which is the MN-major layout, and a block of 128 rows x 8 channels,
+// 16 bytes a row, is a column of its core matrices. M = 128 takes the tile shifted
+// to eight of the nine (dz, dy) offsets (16 channels each), a second M tile the
+// ninth and a block of ones (the bias); N = 48 takes dz for the three dx, shifted
+// the other way: sum_q x[q + off][ci] dz[q - dx][co]. Rows outside the grid are
+// zero in dz and the first and last rows are halo, so every shifted sum is whole.
+// What bounds it: a block of rows costs 49 KB of copies, ~1 us of this SM's share
+// of L2, and beside them 16 MMAs (M = 128, N = 48, K = 16), 0.6 us. One CTA a SM
+// walks its share of the blocks through a ring of WG_STAGES stages (two warps a
+// stage copy with cp.async, one thread issues MMAs; by TMA, whose 16-byte rows are
+// slow, 31 us), keeps its six accumulators in TMEM to the end, and writes one
+// partial; the partials are added in a fixed order. 25 us for 8 x 34^3 rows, the
+// reduction included, where a scalar loop over the rows, which read both operands
+// again for each tap, took 1420 us.
+constexpr int WG_STAGES = 4;
+constexpr int WG_THREADS = 32 * (2 * WG_STAGES + 1);   // two warps copy a stage, one thread issues MMAs
+constexpr int WG_BLOCK = 2 * ROWS * 16;              // 128 rows x 16 channels: 4096
+constexpr int WG_OFF_ONES = 9 * WG_BLOCK;            // after the nine shifted blocks
+constexpr int WG_OFF_DZ = WG_OFF_ONES + WG_BLOCK;
+constexpr int WG_STAGE = WG_OFF_DZ + 3 * WG_BLOCK;   // 53248: dz shifted by dx = -1, 0, 1
+// the second M tile reads 16 half blocks from the ninth on; all but the first
+// four are ignored, but have to lie in shared memory
+constexpr int WG_OFF_BAR = WG_STAGES * WG_STAGE + 12288;
+constexpr int WG_SMEM = WG_OFF_BAR + 128 + 128;
+static_assert(WG_STAGE % 128 == 0 && (WG_STAGES - 1) * WG_STAGE + 8 * WG_BLOCK + 16 * 2048 <= WG_OFF_BAR &&
+              WG_SMEM <= 227 * 1024, "layout");
+// FP32 accumulator, BF16 A and B, both MN-major, N = 48, M = 128
+constexpr uint32_t IDESC_WGRAD =
+    (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((48u >> 3) << 17) | ((128u >> 4) << 24);
+
+struct WgradParams {
+    long long nblocks;       // blocks of 128 rows
+    long long base_row, total_rows;
+    int off9[9];             // row offset of each (dz, dy)
+    const __nv_bfloat16* x;  // padded rows, margin included
+    const __nv_bfloat16* dz;
+    float* partial;          // [CTAs][28][16][16]
+};
+
+// ALIGNED: both operands on 16-byte boundaries (any allocation of their own)
+template <bool ALIGNED>
+__device__ __forceinline__ void copy8(void* dst, const __nv_bfloat16* src) {
+    if constexpr (ALIGNED) {
+        copy16(dst, src);
+    } else {
+        __align__(16) __nv_bfloat16 v[8];
 #pragma unroll
-            for (int c = 0; c < 16; ++c)
-                P.outf[q * 16 + c] = interior ? v[c] + (P.mode == 1 ? P.bias[c] : 0.f) : 0.f;
+        for (int c = 0; c < 8; ++c) v[c] = src[c];
+        *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(v);
+    }
+}
+
+template <bool ALIGNED>
+__global__ void __launch_bounds__(WG_THREADS) weight_grad_kernel(const __grid_constant__ WgradParams P) {
+    extern __shared__ __align__(128) unsigned char raw[];
+    unsigned char* sm = raw + ((128u - (sa(raw) & 127u)) & 127u);
+    uint64_t* full = reinterpret_cast<uint64_t*>(sm + WG_OFF_BAR);
+    uint64_t* empty = full + WG_STAGES;
+    uint64_t* done = empty + WG_STAGES;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
+    volatile int* s_ok = reinterpret_cast<int*>(done + 2);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const long long b0 = P.nblocks * blockIdx.x / gridDim.x, b1 = P.nblocks * (blockIdx.x + 1) / gridDim.x;
+    const int n = (int)(b1 - b0);
+
+    if (tid == 0) {
+        for (int s = 0; s < WG_STAGES; ++s) {
+            mbar_init(&full[s], 64);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(done, 1);
+        fence_mbar_init();
+        *s_ok = 1;
+    }
+    // the block of ones: channel 0 of every row
+    if (tid < ROWS)
+        for (int s = 0; s < WG_STAGES; ++s) {
+            uint4* o = reinterpret_cast<uint4*>(sm + s * WG_STAGE + WG_OFF_ONES);
+            o[tid] = make_uint4(0x3f80u, 0u, 0u, 0u);
+            o[ROWS + tid] = make_uint4(0u, 0u, 0u, 0u);
+        }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (warp == 0) tmem_alloc(tslot, 128);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+
+    if (warp < 2 * WG_STAGES) {
+        // copies: two warps' stage, again and again, once the MMAs have read it
+        const int s = warp >> 1, half = tid & 1;
+        unsigned char* st = sm + s * WG_STAGE + half * (ROWS * 16);
+        uint32_t parity = 1u;
+        for (int i = s; i < n; i += WG_STAGES, parity ^= 1u) {
+            if (!mbar_wait(&empty[s], parity)) {  // (at once the first time)
+                *s_ok = 0;
+                break;
+            }
+            const long long row = P.base_row + (b0 + i) * ROWS;
+            // (rows beyond the allocation, of a last block, meet dz's zeros)
+            for (int k = (tid & 63) >> 1; k < ROWS; k += 32) {
+#pragma unroll
+                for (int r = 0; r < 9; ++r)
+                    copy8<ALIGNED>(st + r * WG_BLOCK + k * 16,
+                                   P.x + min(row + P.off9[r] + k, P.total_rows - 1) * 16 + half * 8);
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    copy8<ALIGNED>(st + WG_OFF_DZ + d * WG_BLOCK + k * 16,
+                                   P.dz + min(row + 1 - d + k, P.total_rows - 1) * 16 + half * 8);
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mbar_arrive(&full[s]);
+        }
+    } else if (lane == 0) {
+        for (int i = 0; i < n; ++i) {
+            const int s = i % WG_STAGES;
+            if (!mbar_wait(&full[s], (uint32_t)(i / WG_STAGES) & 1u)) {
+                *s_ok = 0;
+                break;
+            }
+            tc_fence_after();
+            // MN-major: LBO between groups of 8 rows, SBO between halves
+            const uint64_t ad = smem_desc(sa(sm + s * WG_STAGE), 128, ROWS * 16);
+#pragma unroll
+            for (int k = 0; k < ROWS / 16; ++k)
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+                    umma_f16(tmem + 48 * m, ad + (m * 8 * WG_BLOCK + k * 256) / 16, ad + (WG_OFF_DZ + k * 256) / 16,
+                             IDESC_WGRAD, i > 0 || k > 0);
+            umma_commit(&empty[s]);
+        }
+        umma_commit(done);
+    }
+    __syncthreads();
+    // every thread: the last MMAs have completed
+    if (!mbar_wait(done, 0)) *s_ok = 0;
+    __syncthreads();
+    tc_fence_after();
+    const bool ok = *s_ok;
+    float* part = P.partial + (size_t)blockIdx.x * (TAPS + 1) * 256;
+    if (warp < 4) {
+        for (int dx = 0; dx < 3; ++dx) {
+            float v[16];
+            tmem_ld16(tmem + 16 * dx + ((uint32_t)(32 * warp) << 16), v);
+            const int m = 32 * warp + lane, t = 3 * (m >> 4) + dx, ci = m & 15;
+            float* d = part + (t * 16 + ci) * 16;
+            // a wait that gave up shows as NaN
+#pragma unroll
+            for (int c = 0; c < 16; ++c) d[c] = ok ? v[c] : NAN;
+            if (warp == 0) {
+                tmem_ld16(tmem + 48 + 16 * dx, v);
+                // the ninth offset; then, with dx = 0, the ones' channel 0
+                float* e = lane < 16 ? part + ((24 + dx) * 16 + lane) * 16 : part + TAPS * 256 + (lane - 16) * 16;
+                if (lane < 16 || dx == 1)
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) e[c] = ok ? v[c] : NAN;
+            }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, 32);
+    if (warp == 0) tmem_dealloc(tmem, 128);
 }
 
-// dW[t][ci][co] (+ db[co] as t = 27) partial sums over one chunk of rows:
-// sum over interior rows q of x[q + off_t][ci] * dz[q][co]
-constexpr int WG_ROWS = 1024;
-__global__ void __launch_bounds__(256) weight_grad_kernel(const __nv_bfloat16* x, const __nv_bfloat16* dz,
-                                                          long long rows, long long base_row,
-                                                          const int* taps_off, float* partial) {
-    const int t = blockIdx.y;  // 0..27 (27 = bias)
-    const long long q0 = (long long)blockIdx.x * WG_ROWS;
-    const int ci = threadIdx.x >> 4, co = threadIdx.x & 15;
-    float acc = 0.f;
-    const int off = t < TAPS ? taps_off[t] : 0;
-    for (int i = 0; i < WG_ROWS; ++i) {
-        const long long q = q0 + i;
-        if (q >= rows) break;
-        const float g = __bfloat162float(dz[(base_row + q) * 16 + co]);  // zero on the halo
-        const float a = t < TAPS ? __bfloat162float(x[(base_row + q + off) * 16 + ci]) : (ci == 0 ? 1.f : 0.f);
-        acc = fmaf(a, g, acc);
+// grad[t][ci][co]: the CTAs' partials in a fixed order, eight threads a result
+// with every eighth partial each
+__global__ void __launch_bounds__(256) weight_grad_reduce_kernel(const float* partial, int parts, float* grad) {
+    __shared__ float s[8][33];
+    const int k = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int at = blockIdx.x * 32 + k;
+    float t = 0.f;
+#pragma unroll 4
+    for (int c = g; c < parts; c += 8) t += partial[(size_t)c * (TAPS + 1) * 256 + at];
+    s[g][k] = t;
+    __syncthreads();
+    if (g == 0) {
+        for (int q = 1; q < 8; ++q) t += s[q][k];
+        grad[at] = t;
     }
-    partial[((long long)blockIdx.x * (TAPS + 1) + t) * 256 + threadIdx.x] = acc;
-}
-
-// fixed-order sum of the chunk partials: grad[t][ci][co]
-__global__ void weight_grad_reduce_kernel(const float* partial, int nchunks, float* grad) {
-    const int t = blockIdx.x, k = threadIdx.x;
-    float s = 0.f;
-    for (int c = 0; c < nchunks; ++c) s += partial[((long long)c * (TAPS + 1) + t) * 256 + k];
-    grad[t * 256 + k] = s;
 }
 
 // AdamW on FP32 master parameters
@@ -369,17 +635,11 @@ __global__ void pack_weights_kernel(const float* w, unsigned char* fwd, unsigned
     reinterpret_cast<__nv_bfloat16*>(dgrad + (TAPS - 1 - t) * 512 + (co >> 3) * 256 + ci * 16)[co & 7] = b;
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 encoder() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    if (!fn) {
-        cudaDriverEntryPointQueryResult q;
-        void* p = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    }
-    return fn;
+// CTAs of the persistent kernels: one a SM, at most one a block of rows
+int row_ctas(long long rows) {
+    int dev = 0, sms = 152;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return (int)std::max<long long>(1, std::min<long long>(sms, (rows + ROWS - 1) / ROWS));
 }
 
 }  // namespace
@@ -400,6 +660,7 @@ int bt_conv3d(const bt_conv3d_args* a, void* stream) {
     if ((a->mode == 1 || a->mode == 3) && !a->outf) return BT_E_ARG;
     if ((a->mode == 0 || a->mode == 1) && !a->bias) return BT_E_ARG;
     if (a->mode == 2 && !a->pre) return BT_E_ARG;
+    if (((uintptr_t)a->x | (uintptr_t)a->wpack) & 15u) return BT_E_CUDA;  // 16-byte copies
     const int xp = a->nx + 2, yp = a->ny + 2, zp = a->nz + 2;
     ConvParams P{};
     P.xp = xp;
@@ -407,10 +668,23 @@ int bt_conv3d(const bt_conv3d_args* a, void* stream) {
     P.zp = zp;
     P.rows = (long long)a->nb * xp * yp * zp;
     P.base_row = bt_conv3d_margin(a->nx, a->ny);
-    int t = 0;
-    for (int dz = -1; dz <= 1; ++dz)
-        for (int dy = -1; dy <= 1; ++dy)
-            for (int dx = -1; dx <= 1; ++dx) P.taps_off[t++] = dz * xp * yp + dy * xp + dx;
+    const bool by_plane = 3 * (ROWS + 2 * (xp + 1)) <= A_ROWS;
+    P.nwin = by_plane ? 3 : 9;
+    P.win_rows = by_plane ? ROWS + 2 * (xp + 1) : WIN_ROWS;
+    for (int w = 0; w < P.nwin; ++w)
+        P.win_off[w] = by_plane ? (w - 1) * xp * yp - xp - 1 : (w / 3 - 1) * xp * yp + (w % 3 - 1) * xp - 1;
+    for (int t = 0; t < TAPS; ++t)  // t = (dz + 1) * 9 + (dy + 1) * 3 + (dx + 1)
+        P.tap_row[t] = by_plane ? (t / 9) * P.win_rows + (t / 3 % 3) * xp + t % 3 : (t / 3) * WIN_ROWS + t % 3;
+    P.half = (P.nwin * P.win_rows * 16 + 127) / 128 * 128;
+    P.stages = std::min(CONV_STAGES, CONV_ROOM / (2 * P.half));
+    P.x = (const __nv_bfloat16*)a->x;
+    P.total_rows = P.rows + 2 * P.base_row;
+    if (P.rows < (1LL << 31)) {
+        P.by_xp = bt::make_fast_div((uint32_t)xp);
+        P.by_plane = bt::make_fast_div((uint32_t)(xp * yp));
+        P.by_sample = bt::make_fast_div((uint32_t)(xp * yp * zp));
+    }
+    P.vec = (((uintptr_t)a->pre | (uintptr_t)a->outf) & 15u) == 0;
     P.wpack = (const unsigned char*)a->wpack;
     P.bias = a->bias;
     P.mode = a->mode;
@@ -418,27 +692,13 @@ int bt_conv3d(const bt_conv3d_args* a, void* stream) {
     P.pre = a->pre;
     P.outf = a->outf;
     P.status = a->status;
-    // 2-D view of the whole allocation: 16 channels x (rows + 2 margins)
-    auto fn = encoder();
-    if (!fn) return BT_E_CUDA;
-    CUtensorMap map;
-    const cuuint64_t total_rows = (cuuint64_t)(P.rows + 2 * P.base_row);
-    cuuint64_t dims[2] = {16, total_rows};
-    cuuint64_t strides[1] = {32};
-    cuuint32_t box[2] = {8, ROWS};
-    cuuint32_t es[2] = {1, 1};
-    if (fn(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(a->x), dims, strides, box, es,
-           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return BT_E_CUDA;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(conv3d_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CONV_SMEM) != cudaSuccess)
             return BT_E_CUDA;
         configured = true;
     }
-    const long long nblocks = (P.rows + ROWS - 1) / ROWS;
-    conv3d_kernel<<<(unsigned)nblocks, 128, CONV_SMEM, (cudaStream_t)stream>>>(P, map);
+    conv3d_kernel<<<row_ctas(P.rows), CONV_THREADS, CONV_SMEM, (cudaStream_t)stream>>>(P);
     return cudaGetLastError() == cudaSuccess ? BT_OK : BT_E_CUDA;
 }
 
@@ -453,26 +713,28 @@ int bt_conv3d_weight_grad(const void* x, const void* dz, int nb, int nx, int ny,
     if (!x || !dz || !partial || !grad || nb <= 0) return BT_E_ARG;
     const int xp = nx + 2, yp = ny + 2, zp = nz + 2;
     const long long rows = (long long)nb * xp * yp * zp;
-    int offs[TAPS];
-    int t = 0;
-    for (int dzz = -1; dzz <= 1; ++dzz)
-        for (int dy = -1; dy <= 1; ++dy)
-            for (int dx = -1; dx <= 1; ++dx) offs[t++] = dzz * xp * yp + dy * xp + dx;
-    // the offsets travel in the partial buffer's tail (caller sizes it with bt_conv3d_wgrad_scratch)
-    const int nchunks = (int)((rows + WG_ROWS - 1) / WG_ROWS);
-    int* d_offs = reinterpret_cast<int*>(partial + (size_t)nchunks * (TAPS + 1) * 256);
+    WgradParams P{};
+    P.nblocks = (rows + ROWS - 1) / ROWS;
+    P.base_row = bt_conv3d_margin(nx, ny);
+    for (int r = 0; r < 9; ++r) P.off9[r] = (r / 3 - 1) * xp * yp + (r % 3 - 1) * xp;
+    P.partial = partial;
+    P.x = (const __nv_bfloat16*)x;
+    P.dz = (const __nv_bfloat16*)dz;
+    P.total_rows = rows + 2 * P.base_row;
     cudaStream_t s = (cudaStream_t)stream;
-    if (cudaMemcpyAsync(d_offs, offs, sizeof(offs), cudaMemcpyHostToDevice, s) != cudaSuccess) return BT_E_CUDA;
-    weight_grad_kernel<<<dim3(nchunks, TAPS + 1), 256, 0, s>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dz,
-                                                                rows, bt_conv3d_margin(nx, ny), d_offs, partial);
-    weight_grad_reduce_kernel<<<TAPS + 1, 256, 0, s>>>(partial, nchunks, grad);
+    const int ctas = row_ctas(rows);
+    const bool aligned = (((uintptr_t)x | (uintptr_t)dz) & 15u) == 0;
+    auto kernel = aligned ? weight_grad_kernel<true> : weight_grad_kernel<false>;
+    // (set on every call: it is per device)
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM) != cudaSuccess)
+        return BT_E_CUDA;
+    kernel<<<ctas, WG_THREADS, WG_SMEM, s>>>(P);
+    weight_grad_reduce_kernel<<<(TAPS + 1) * 8, 256, 0, s>>>(partial, ctas, grad);
     return cudaGetLastError() == cudaSuccess ? BT_OK : BT_E_CUDA;
 }
 
 long long bt_conv3d_wgrad_scratch(int nb, int nx, int ny, int nz) {
-    const long long rows = (long long)nb * (nx + 2) * (ny + 2) * (nz + 2);
-    const long long nchunks = (rows + WG_ROWS - 1) / WG_ROWS;
-    return nchunks * (TAPS + 1) * 256 + 64;  // floats, + room for the tap offsets
+    return (long long)row_ctas((long long)nb * (nx + 2) * (ny + 2) * (nz + 2)) * (TAPS + 1) * 256;  // floats
 }
 
 int bt_adamw(float* p, const float* g, float* m, float* v, int n, float lr, float beta1, float beta2, float eps,
