@@ -333,7 +333,7 @@ typedef struct bt_conv3d_args {
     const void* x;           /* BF16 padded rows */
     const void* wpack;       /* 27*512 bytes */
     const float* bias;       /* 16 floats (modes 0, 1) */
-    void* out;               /* BF16 padded rows (modes 0, 2); halo rows written as zero */
+    void* out;               /* BF16 padded rows (modes 0, 2); halo and margin rows written as zero */
     float* pre;              /* FP32 rows: written in mode 0 (may be NULL), read in mode 2 */
     float* outf;             /* FP32 rows (modes 1, 3) */
     int* status;             /* device int; bit 8 set when a bounded wait gave up */
@@ -345,8 +345,17 @@ int bt_conv3d(const bt_conv3d_args* a, void* stream);
  * partial: bt_conv3d_wgrad_scratch(...) floats of device scratch. */
 int bt_conv3d_weight_grad(const void* x, const void* dz, int nb, int nx, int ny, int nz, float* partial,
                           float* grad, void* stream);
+/* The same with dL/db[16] in bias_grad and grad[27][16][16] only. */
+int bt_conv3d_weight_bias_grad(const void* x, const void* dz, int nb, int nx, int ny, int nz, float* partial,
+                               float* grad, float* bias_grad, void* stream);
 long long bt_conv3d_wgrad_scratch(int nb, int nx, int ny, int nz);
 int bt_conv3d_pack_weights(const float* w, void* wpack_fwd, void* wpack_dgrad, void* stream);
+/* The weights of several layers, w[layers][27][16][16], in one launch: a layer's
+ * forward block, then its data-gradient block. */
+int bt_conv3d_pack_layers(const float* w, int layers, void* wpack, void* stream);
+/* FP32 rows (no margin) as BF16 padded rows, margins zero; both on 16-byte
+ * boundaries (BT_E_ARG otherwise). */
+int bt_conv3d_pad_rows(const float* rows_f32, int nb, int nx, int ny, int nz, void* out, void* stream);
 /* AdamW on FP32 parameters (step counts from 1). */
 int bt_adamw(float* p, const float* g, float* m, float* v, int n, float lr, float beta1, float beta2, float eps,
              float weight_decay, int step, void* stream);

@@ -74,6 +74,7 @@ EXPORTS = [
     "bt_read_mt_phases", "bt_stream", "bt_measure", "bt_launch_count", "bt_sequence_schedule",
     "bt_version", "bt_autotune", "bt_set_tma_split", "bt_set_tma_chunks", "bt_step_noalloc",
     "bt_conv3d_margin", "bt_conv3d", "bt_conv3d_weight_grad", "bt_conv3d_wgrad_scratch", "bt_conv3d_pack_weights",
+    "bt_conv3d_weight_bias_grad", "bt_conv3d_pack_layers", "bt_conv3d_pad_rows",
     "bt_adamw", "bt_umma_selftest", "bt_field_device", "bt_set_wait_polls",
 ]
 
@@ -124,6 +125,9 @@ def lib():
         "bt_conv3d_margin": ([i, i], ll),
         "bt_conv3d": ([ctypes.POINTER(Conv3dArgs), vp], i),
         "bt_conv3d_weight_grad": ([vp, vp, i, i, i, i, vp, vp, vp], i),
+        "bt_conv3d_weight_bias_grad": ([vp, vp, i, i, i, i, vp, vp, vp, vp], i),
+        "bt_conv3d_pack_layers": ([vp, i, vp, vp], i),
+        "bt_conv3d_pad_rows": ([vp, i, i, i, i, vp, vp], i),
         "bt_conv3d_wgrad_scratch": ([i, i, i, i], ll),
         "bt_conv3d_pack_weights": ([vp, vp, vp, vp], i),
         "bt_adamw": ([vp, vp, vp, vp, i, ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float,

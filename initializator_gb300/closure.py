@@ -33,6 +33,11 @@ class PaddedRows:
         import torch
         return torch.zeros((self.total, CH), dtype=torch.bfloat16, device=device)
 
+    def _unset(self, device):
+        """empty() without the fill, for kernels that write margins and halo too."""
+        import torch
+        return torch.empty((self.total, CH), dtype=torch.bfloat16, device=device)
+
     def pack(self, a, device):
         """a: (nb, nz, ny, nx, C<=16) array or tensor -> padded BF16 rows."""
         import torch
@@ -70,8 +75,8 @@ def conv3d(layout: PaddedRows, x, wpack, mode, bias=None, out=None, pre=None, ou
 def pack_weights(w):
     """w: (27, 16, 16) FP32 CUDA tensor -> (forward, data-gradient) packed BF16 blocks."""
     import torch
-    fwd = torch.zeros(TAPS * 512, dtype=torch.uint8, device=w.device)
-    dg = torch.zeros(TAPS * 512, dtype=torch.uint8, device=w.device)
+    fwd = torch.empty(TAPS * 512, dtype=torch.uint8, device=w.device)
+    dg = torch.empty(TAPS * 512, dtype=torch.uint8, device=w.device)
     rc = lib().bt_conv3d_pack_weights(_ptr(w.contiguous()), _ptr(fwd), _ptr(dg),
                                       ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
     if rc:
@@ -126,7 +131,13 @@ class Net:
         return self.flat[self.NW:].view(4, CH)[i]
 
     def repack(self):
-        self.packed = [pack_weights(self.w(i)) for i in range(4)]
+        import torch
+        buf = torch.empty((4, 2, TAPS * 512), dtype=torch.uint8, device=self.device)
+        rc = lib().bt_conv3d_pack_layers(_ptr(self.flat), 4, _ptr(buf),
+                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        if rc:
+            raise BtError(rc, "bt_conv3d_pack_layers")
+        self.packed = [tuple(layer.unbind()) for layer in buf.unbind()]
 
     def forward(self, layout: PaddedRows, x):
         """x: BF16 padded rows -> FP32 output rows (16 channels), with the
@@ -135,7 +146,7 @@ class Net:
         acts, pres = [x], []
         a = x
         for i in range(3):
-            out = layout.empty(self.device)
+            out = layout._unset(self.device)
             pre = torch.empty((layout.rows, CH), dtype=torch.float32, device=self.device)
             conv3d(layout, a, self.packed[i][0], 0, bias=self.b(i), out=out, pre=pre, status=self.status)
             acts.append(out)
@@ -149,17 +160,28 @@ class Net:
     def backward(self, layout: PaddedRows, dy):
         """dy: FP32 rows (zero on the halo) = dL/dy. Fills self.grad."""
         acts, pres = self._cache
-        g = layout.empty(self.device)
-        g[layout.margin:layout.margin + layout.rows] = dy.to(g.dtype)
+        import torch
+        fn, stream = lib(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        grid = layout.nb, layout.nx, layout.ny, layout.nz
+        if dy.is_cuda and dy.dtype is torch.float32 and dy.shape == (layout.rows, CH) and dy.is_contiguous() and \
+                dy.data_ptr() % 16 == 0:
+            g = layout._unset(self.device)
+            rc = fn.bt_conv3d_pad_rows(_ptr(dy), *grid, _ptr(g), stream)
+            if rc:
+                raise BtError(rc, "bt_conv3d_pad_rows")
+        else:
+            g = layout.empty(self.device)
+            g[layout.margin:layout.margin + layout.rows] = dy.to(g.dtype)
         gw = self.grad[:self.NW].view(4, TAPS, CH, CH)
         gb = self.grad[self.NW:].view(4, CH)
-        scratch = None
+        scratch = torch.empty(int(fn.bt_conv3d_wgrad_scratch(*grid)), dtype=torch.float32, device=g.device)
         for i in range(3, -1, -1):
-            gwi, gbi, scratch = weight_grad(layout, acts[i], g, scratch)
-            gw[i] = gwi
-            gb[i] = gbi
+            rc = fn.bt_conv3d_weight_bias_grad(_ptr(acts[i]), _ptr(g), *grid, _ptr(scratch), _ptr(gw[i]), _ptr(gb[i]),
+                                               stream)
+            if rc:
+                raise BtError(rc, "bt_conv3d_weight_bias_grad")
             if i > 0:
-                nxt = layout.empty(self.device)
+                nxt = layout._unset(self.device)
                 conv3d(layout, g, self.packed[i][1], 2, out=nxt, pre=pres[i - 1], status=self.status)
                 g = nxt
 

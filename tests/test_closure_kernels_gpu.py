@@ -86,3 +86,47 @@ def test_weight_grad_exact(shape, aligned, btlib):
     want_w, want_b = co.conv3d_weight_grad(x, dz)
     np.testing.assert_array_equal(gw.cpu().numpy(), want_w)
     np.testing.assert_array_equal(gb.cpu().numpy(), want_b)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 3, 5, 7), (1, 2, 3, 127)])
+def test_outputs_cover_margins(shape, btlib):
+    """BF16 outputs are whole, margins included, in buffers that held something
+    else: of the convolution and of FP32 rows turned into padded ones; the grouped
+    forms of packing and of the weight gradient give what the single ones give."""
+    import ctypes
+
+    import torch
+    from initializator_gb300 import closure
+    nb, nz, ny, nx = shape
+    rng = np.random.default_rng(nx)
+    lay = closure.PaddedRows(nb, nz, ny, nx)
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    xr = lay.pack(_ints(rng, (nb, nz, ny, nx, 16), 2), "cuda")
+    w = torch.tensor(_ints(rng, (3, 27, 16, 16), 2), dtype=torch.float32, device="cuda")
+    packed = torch.empty((3, 2, 27 * 512), dtype=torch.uint8, device="cuda")
+    assert btlib.bt_conv3d_pack_layers(ptr(w), 3, ptr(packed), stream) == 0
+    for i in range(3):
+        for k, one in enumerate(closure.pack_weights(w[i])):
+            assert torch.equal(packed[i, k], one)
+
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    bias = torch.tensor(_ints(rng, 16, 3), dtype=torch.float32, device="cuda")
+    clean, dirty = lay.empty("cuda"), torch.full_like(lay.empty("cuda"), 3.0)
+    for out in (clean, dirty):
+        closure.conv3d(lay, xr, packed[1, 0], 0, bias=bias, out=out, status=st)
+    assert torch.equal(clean, dirty) and int(st.item()) == 0
+
+    rows = torch.randn((lay.rows, 16), device="cuda")
+    out = torch.full_like(clean, 3.0)
+    assert btlib.bt_conv3d_pad_rows(ptr(rows), nb, nx, ny, nz, ptr(out), stream) == 0
+    want = lay.empty("cuda")
+    want[lay.margin:lay.margin + lay.rows] = rows.to(torch.bfloat16)
+    assert torch.equal(out, want)
+    assert btlib.bt_conv3d_pad_rows(ctypes.c_void_p(rows.data_ptr() + 4), nb, nx, ny, nz, ptr(out), stream) < 0
+
+    gw, gb, scratch = closure.weight_grad(lay, xr, clean)
+    both = torch.full((27 * 256 + 16 + 1,), 5.0, device="cuda")
+    assert btlib.bt_conv3d_weight_bias_grad(ptr(xr), ptr(clean), nb, nx, ny, nz, ptr(scratch), ptr(both),
+                                            ptr(both[27 * 256:]), stream) == 0
+    assert torch.equal(both[:27 * 256], gw.flatten()) and torch.equal(both[27 * 256:-1], gb) and float(both[-1]) == 5.0
