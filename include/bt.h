@@ -278,13 +278,12 @@ int bt_field_device(bt_handle* h, int member, void** mx, void** my, void** mz, i
 long long bt_launch_count(const bt_handle* h);
 
 /* Limits of bt_step_noalloc: its scratch is a fixed array compiled into the
- * library (about 2.4 MB on every device that loads it). */
+ * library (58 KB on every device that loads it). */
 #define BT_NOALLOC_MAX_VOXELS (1 << 21)   /* nx*ny*nz, e.g. 128^3 */
-#define BT_NOALLOC_MAX_BLOCKS 16384       /* CTAs of the step kernel's grid */
+#define BT_NOALLOC_MAX_BLOCKS 16384       /* column tiles of 32 x 8 x (a share of nz) */
 
-/* One step of the REFERENCE-scheme update (the fused kernel bt_run uses for
- * FP64 and for the FP32 steps the fast path does not take) that performs no
- * device allocation. No
+/* One step of the REFERENCE-scheme update (the arithmetic of the kernels bt_run
+ * uses for FP64) that performs no device allocation. No
  * counterpart in the reference: it exists for callers that may not call
  * cudaMalloc — code running under CUDA stream capture, hosts whose framework
  * has reserved the device's memory for its own pool, plugin hosts that forbid
@@ -297,9 +296,8 @@ long long bt_launch_count(const bt_handle* h);
  * cfg->batch must be 0 or 1, cfg->velocity 0 or 1 and cfg->boundary all
  * BT_BC_COPY (BT_E_ARG otherwise).
  * Asynchronous on `stream` (a cudaStream_t, NULL = legacy default stream).
- * The scratch (run control, schedule record, per-CTA partial sums, geometry
- * code) is one file-scope __device__ array shared by every call on a device
- * and keeping the last call's contents; each call re-initialises it, so calls
+ * The scratch (per-CTA partial sums) is one file-scope __device__ array shared
+ * by every call on a device; each call writes what it reads, so calls
  * ordered on one stream are independent, but calls that overlap on the GPU
  * race and must not be issued. The first call on a device (and the first
  * after its context was reset) looks up the array's device address

@@ -206,6 +206,11 @@ template <typename T>
 cudaError_t launch_step(const StepParams<T>& p, int scheme, int vel, int prec, dim3 grid, cudaStream_t s);
 template <typename T>
 cudaError_t launch_sums(const StepParams<T>& p, double* out4, cudaStream_t s);
+// one step over dense arrays straight from the mask (sets p's list fields;
+// p.partials: 3 SINGLE_CTAS doubles)
+template <typename T>
+cudaError_t launch_single(StepParams<T>& p, const uint8_t* mask, const double grad[3], int vel, int prec, cudaStream_t s);
+constexpr int SINGLE_CTAS = 16 * 152;  // at most
 // MacCormack step (predictor into pred, then corrector into p.out)
 template <typename T>
 cudaError_t launch_mac(const StepParams<T>& p, T* const pred[3], int vel, int prec, dim3 grid, cudaStream_t s);

@@ -9,20 +9,18 @@
 // caller owns every input and output buffer and passes them in; this entry
 // point needs no handle and allocates nothing.
 //
-// The step itself is the library's generic fused kernel (step_kernel in
-// bt_step.cuh, the same code the handle-based API runs for FP64 and for steps
-// that carry pulses). Its scratch — the run-control block (step counter, CTA
-// ticket), the per-step schedule record, the per-CTA partial sums of M(t) and
-// the per-voxel geometry code derived from the mask — lives in the file-scope
-// array below instead of in memory allocated by bt_create. Every GPU that
-// loads the library holds that array until the process exits.
+// The step itself is the library's generic update (single_step_kernel,
+// bt_step_single.cuh: the arithmetic of the kernels that the handle-based API
+// runs for FP64 and for steps that carry pulses). Its scratch, the per-CTA sums
+// of M(t), lives in the file-scope array below instead of in memory allocated by
+// bt_create. Every GPU that loads the library holds that array until the process
+// exits.
 //
-// Sharing: all calls on a device use the same array, and the array keeps the
-// previous call's contents. Each call clears what must start at zero (the
-// run-control block) and rebuilds the rest before its step kernel reads it,
-// so sequential calls are independent. Calls whose kernels overlap on the GPU
-// (different streams, or different host threads, without ordering between
-// them) race on the array and give wrong results: order them on one stream.
+// Sharing: all calls on a device use the same array. Each call writes what its
+// second kernel reads, so sequential calls are independent. Calls whose kernels
+// overlap on the GPU (different streams, or different host threads, without
+// ordering between them) race on the array and give wrong results: order them on
+// one stream.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -36,17 +34,9 @@
 
 namespace {
 
-constexpr size_t OFF_CTL = 0;                                     // bt::Ctl
-constexpr size_t OFF_STEP = 256;                                  // one bt::StepInfo
-constexpr size_t OFF_PULSE = 768;                                 // one bt::DevPulse
-constexpr size_t OFF_PARTIALS = 1024;                             // 3 doubles per CTA
-constexpr size_t OFF_CODE = OFF_PARTIALS + 3 * sizeof(double) * BT_NOALLOC_MAX_BLOCKS;
-constexpr size_t SCRATCH_BYTES = OFF_CODE + BT_NOALLOC_MAX_VOXELS;
-static_assert(sizeof(bt::Ctl) <= OFF_STEP - OFF_CTL, "layout");
-static_assert(sizeof(bt::StepInfo) <= OFF_PULSE - OFF_STEP, "layout");
-static_assert(sizeof(bt::DevPulse) <= OFF_PARTIALS - OFF_PULSE, "layout");
+constexpr size_t SCRATCH_BYTES = 3 * sizeof(double) * bt::SINGLE_CTAS;
 
-// The scratch of every allocation-free call on this device (about 2.4 MB).
+// The scratch of every allocation-free call on this device (58 KB).
 static __device__ __align__(256) unsigned char g_noalloc_scratch[SCRATCH_BYTES];
 
 constexpr int MAX_DEVICES = 64;
@@ -109,58 +99,16 @@ cudaError_t scratch_for_current_device(cudaStream_t stream, unsigned char** out)
     return cudaSuccess;
 }
 
-// the geometry code of the kernels (bit f: in-domain solid face neighbour
-// -x,+x,-y,+y,-z,+z; bit 6: pore) from a dense mask, into the scratch array
-__global__ void noalloc_code_kernel(const uint8_t* mask, uint8_t* code, int nx, int ny, int nz) {
-    const long long n = (long long)nx * ny * nz;
-    const long long plane = (long long)nx * ny;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(q % nx), y = (int)((q / nx) % ny), z = (int)(q / plane);
-        uint8_t c = 0;
-        if (mask[q]) {
-            c = bt::CODE_PORE;
-            if (x > 0 && !mask[q - 1]) c |= 1;
-            if (x < nx - 1 && !mask[q + 1]) c |= 2;
-            if (y > 0 && !mask[q - nx]) c |= 4;
-            if (y < ny - 1 && !mask[q + nx]) c |= 8;
-            if (z > 0 && !mask[q - plane]) c |= 16;
-            if (z < nz - 1 && !mask[q + plane]) c |= 32;
-        }
-        code[q] = c;
-    }
-}
-
-// the schedule record of the single step: static gradient, no pulses
-__global__ void noalloc_step_record_kernel(bt::StepInfo* si, bt::DevPulse* pu, double gx, double gy, double gz) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    si->grad[0] = gx;
-    si->grad[1] = gy;
-    si->grad[2] = gz;
-    for (int a = 0; a < 3; ++a) si->knext[a] = 0.0;
-    for (int f = 0; f < 6; ++f) {
-        si->phase[f][0] = 1.0;
-        si->phase[f][1] = 0.0;
-    }
-    si->pulse_first = 0;
-    si->pulse_count = 0;
-    pu->flag = 0;
-}
-
 template <typename T>
 void fill(const bt_config& c, bt::StepParams<T>& P, const void* const in[3], void* const out[3], const void* vx,
-          const void* vy, const void* vz, unsigned char* scratch, double* sums, dim3 grid) {
+          const void* vy, const void* vz, unsigned char* scratch, double* sums) {
     constexpr double SMALL = 1.0e-50;
     std::memset(&P, 0, sizeof(P));
     P.nx = c.nx; P.ny = c.ny; P.nz = c.nz;
-    P.pitch = c.nx; P.vxpitch = c.nx + 1; P.cpitch = c.nx;   // the caller's dense layouts
-    P.plane = (long long)c.nx * c.ny;
-    P.zsplit = (int)grid.z;
-    P.zchunk = (c.nz + P.zsplit - 1) / P.zsplit;
     for (int k = 0; k < 3; ++k) {
         P.in[k] = static_cast<const T*>(in[k]);
         P.out[k] = static_cast<T*>(out[k]);
     }
-    P.code = scratch + OFF_CODE;
     P.vx = static_cast<const T*>(vx);
     P.vy = static_cast<const T*>(vy);
     P.vz = static_cast<const T*>(vz);
@@ -197,14 +145,9 @@ void fill(const bt_config& c, bt::StepParams<T>& P, const void* const in[3], voi
     P.box[0] = c.buffer[0]; P.box[1] = c.nx - c.buffer[0];
     P.box[2] = c.buffer[1]; P.box[3] = c.ny - c.buffer[1];
     P.box[4] = c.buffer[2]; P.box[5] = c.nz - c.buffer[2];
-    P.dxd = c.dx; P.dyd = c.dy; P.dzd = c.dz; P.gamma = c.gamma;
-    P.steps = reinterpret_cast<const bt::StepInfo*>(scratch + OFF_STEP);
-    P.nsched = 0;  // steps[0] is the record written by this call
-    P.pulses = reinterpret_cast<const bt::DevPulse*>(scratch + OFF_PULSE);
-    P.ctl = reinterpret_cast<bt::Ctl*>(scratch + OFF_CTL);
-    P.partials = reinterpret_cast<double*>(scratch + OFF_PARTIALS);
+    P.dxd = c.dx; P.dyd = c.dy; P.dzd = c.dz;
+    P.partials = reinterpret_cast<double*>(scratch);
     P.mt = sums;
-    P.mt_cap = 1;
 }
 
 }  // namespace
@@ -234,8 +177,8 @@ extern "C" int bt_step_noalloc(const bt_config* cfg, const uint8_t* mask, const 
                      c.nx, c.ny, c.nz, nvox, BT_NOALLOC_MAX_VOXELS);
         return BT_E_SIZE;
     }
-    // the generic kernel's grid: 32 x 8 column tiles, z split to fill the SMs,
-    // no empty z-chunk
+    // the grid's size in column tiles of 32 x 8, z split to fill the SMs, no empty
+    // z-chunk: a caller's limit
     const int gx = (c.nx + bt::TX - 1) / bt::TX, gy = (c.ny + bt::TY - 1) / bt::TY;
     const long long tiles = (long long)gx * gy;
     int zsplit = 1;
@@ -249,7 +192,6 @@ extern "C" int bt_step_noalloc(const bt_config* cfg, const uint8_t* mask, const 
                      tiles * zsplit, BT_NOALLOC_MAX_BLOCKS);
         return BT_E_SIZE;
     }
-    const dim3 grid(gx, gy, zsplit);
     unsigned char* scratch = nullptr;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const cudaError_t se = scratch_for_current_device(s, &scratch);
@@ -260,13 +202,6 @@ extern "C" int bt_step_noalloc(const bt_config* cfg, const uint8_t* mask, const 
         return BT_E_ARG;
     }
     if (se != cudaSuccess) return BT_E_CUDA;
-    // the run-control block must start at zero (step 0, no ticket, no status)
-    if (cudaMemsetAsync(scratch + OFF_CTL, 0, sizeof(bt::Ctl), s) != cudaSuccess) return BT_E_CUDA;
-    noalloc_step_record_kernel<<<1, 32, 0, s>>>(reinterpret_cast<bt::StepInfo*>(scratch + OFF_STEP),
-                                                reinterpret_cast<bt::DevPulse*>(scratch + OFF_PULSE), c.grad[0],
-                                                c.grad[1], c.grad[2]);
-    noalloc_code_kernel<<<1216, 256, 0, s>>>(mask, scratch + OFF_CODE, c.nx, c.ny, c.nz);
-    if (cudaGetLastError() != cudaSuccess) return BT_E_CUDA;
     const void* in[3] = {mx_in, my_in, mz_in};
     void* out[3] = {mx_out, my_out, mz_out};
     const int prec = c.vector_mult == 1 ? 1 : 0;
@@ -274,12 +209,12 @@ extern "C" int bt_step_noalloc(const bt_config* cfg, const uint8_t* mask, const 
     cudaError_t e;
     if (c.precision == BT_F64) {
         bt::StepParams<double> P;
-        fill<double>(c, P, in, out, vx, vy, vz, scratch, sums, grid);
-        e = bt::launch_step<double>(P, BT_SCHEME_REFERENCE, vel, prec, grid, s);
+        fill<double>(c, P, in, out, vx, vy, vz, scratch, sums);
+        e = bt::launch_single<double>(P, mask, c.grad, vel, prec, s);
     } else {
         bt::StepParams<float> P;
-        fill<float>(c, P, in, out, vx, vy, vz, scratch, sums, grid);
-        e = bt::launch_step<float>(P, BT_SCHEME_REFERENCE, vel, prec, grid, s);
+        fill<float>(c, P, in, out, vx, vy, vz, scratch, sums);
+        e = bt::launch_single<float>(P, mask, c.grad, vel, prec, s);
     }
     return e == cudaSuccess ? BT_OK : BT_E_CUDA;
 }

@@ -5,12 +5,18 @@
 #include "bt_step_tma.cuh"
 #include "bt_step_mac.cuh"
 #include "bt_step_pore.cuh"
+#include "bt_step_single.cuh"
 
 namespace bt {
 
 template <>
 cudaError_t launch_step<float>(const StepParams<float>& p, int scheme, int vel, int prec, dim3 grid, cudaStream_t s) {
     return launch_step_impl<float>(p, scheme, vel, prec, grid, s);
+}
+
+template <>
+cudaError_t launch_single<float>(StepParams<float>& p, const uint8_t* mask, const double grad[3], int vel, int prec, cudaStream_t s) {
+    return launch_single_impl<float>(p, mask, grad, vel, prec, s);
 }
 
 template <>

@@ -4,12 +4,18 @@
 #include "bt_step.cuh"
 #include "bt_step_mac.cuh"
 #include "bt_step_pore.cuh"
+#include "bt_step_single.cuh"
 
 namespace bt {
 
 template <>
 cudaError_t launch_step<double>(const StepParams<double>& p, int scheme, int vel, int prec, dim3 grid, cudaStream_t s) {
     return launch_step_impl<double>(p, scheme, vel, prec, grid, s);
+}
+
+template <>
+cudaError_t launch_single<double>(StepParams<double>& p, const uint8_t* mask, const double grad[3], int vel, int prec, cudaStream_t s) {
+    return launch_single_impl<double>(p, mask, grad, vel, prec, s);
 }
 
 template <>

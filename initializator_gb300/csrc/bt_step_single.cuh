@@ -1,0 +1,127 @@
+// One step over dense arrays of the caller's, straight from its mask
+// (bt_step_noalloc): a voxel a thread, then the sums of the CTAs.
+//
+// What bounds it: latency. A grid that one call steps once has a few voxels a
+// lane of the GPU and fits in L2; four launches, the memset of the run control,
+// the schedule record, the geometry code and the dense z-march with its two
+// barriers a plane and the ticket, took 35 us for 48^3 voxels (FP32). The faces' bits
+// come from the mask's neighbours here, the gradient is an argument, and the
+// second kernel, one CTA launched as a programmatic dependent, adds the CTAs'
+// sums: no state is left between calls. Now 6.8 us of a replayed graph a call, 8 us
+// a call from C in a loop.
+#pragma once
+#include "bt_step_pore.cuh"
+
+namespace bt {
+
+// CTAs: one a 128 voxels, at most 16 a SM (their sums are added by one CTA)
+template <typename T, bool VEL, bool PREC>
+__global__ void __launch_bounds__(PT) single_step_kernel(const __grid_constant__ StepParams<T> P, const uint8_t* __restrict__ mask,
+                                                         double3 grad) {
+    __shared__ double sums[3][PT];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int nx = P.nx, ny = P.ny, nz = P.nz;
+    const int plane = nx * ny, n = plane * nz;
+    T gd[3] = {0, 0, 0};
+    if constexpr (PREC) {
+        gd[0] = (T)(grad.x * P.dxd);
+        gd[1] = (T)(grad.y * P.dyd);
+        gd[2] = (T)(grad.z * P.dzd);
+    }
+    Acc<T> acc[3];
+    for (int q = blockIdx.x * PT + threadIdx.x; q < n; q += gridDim.x * PT) {
+        const Cell v = cell_of((uint32_t)q, P.by_pitch, P.by_ny, nx, ny);
+        T o[3] = {0, 0, 0};
+        if (mask[q]) {
+            const bool open[6] = {v.x > 0, v.x < nx - 1, v.y > 0, v.y < ny - 1, v.z > 0, v.z < nz - 1};
+            T p0[3], nb[3][6];
+            load_neighbours<T>(P.in, (uint32_t)q, open, nx, plane, p0, nb);
+            // bit a: a solid neighbour inside the domain
+            const int at[6] = {open[0] ? q - 1 : q,  open[1] ? q + 1 : q,     open[2] ? q - nx : q,
+                               open[3] ? q + nx : q, open[4] ? q - plane : q, open[5] ? q + plane : q};
+            int f = 0;
+#pragma unroll
+            for (int a = 0; a < 6; ++a) f |= mask[at[a]] ? 0 : 1 << a;
+            T vf[6] = {0, 0, 0, 0, 0, 0};
+            if constexpr (VEL) {
+                const T* vx = P.vx + (v.z * ny + v.y) * (nx + 1) + v.x;
+                const T* vy = P.vy + (v.z * (ny + 1) + v.y) * nx + v.x;
+                vf[0] = vx[0];
+                vf[1] = vx[1];
+                vf[2] = vy[0];
+                vf[3] = vy[nx];
+                vf[4] = P.vz[q];
+                vf[5] = P.vz[q + plane];
+            }
+            T df[6];
+#pragma unroll
+            for (int a = 0; a < 6; ++a) df[a] = (f & (1 << a)) ? P.dps : P.dpp;
+            T bb[3] = {0, 0, 0};
+            if constexpr (PREC) {
+                bb[0] = P.b * (gd[0] * ((T)v.x + (T)0.5));
+                bb[1] = P.b * (gd[1] * ((T)v.y + (T)0.5));
+                bb[2] = P.b * (gd[2] * ((T)v.z + (T)0.5));
+            }
+            voxel_step<T, SCHEME_REF, VEL, PREC>(P, p0, nb, P.dtt1[f], P.dtt2[f], vf, df, bb, o);
+            if (v.x >= P.box[0] && v.x < P.box[1] && v.y >= P.box[2] && v.y < P.box[3] && v.z >= P.box[4] && v.z < P.box[5])
+#pragma unroll
+                for (int c = 0; c < 3; ++c) acc[c].add(o[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) P.out[c][q] = o[c];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        if constexpr (sizeof(T) == 8) sums[c][threadIdx.x] = acc[c].s;
+        else reinterpret_cast<float2*>(sums[c])[threadIdx.x] = make_float2(acc[c].s, -acc[c].c);
+    }
+    chunk_sums<T, 3>(P, 0, blockIdx.x, sums);
+}
+
+// the CTAs' sums in a fixed order (one CTA)
+template <typename T>
+__global__ void __launch_bounds__(256) single_finish_kernel(const double* parts, int n, double* out) {
+    __shared__ double sums[8][3];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    double t[3] = {0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int q = tid; q < n; q += 256)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) t[c] += __ldcg(&parts[3 * q + c]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t[c] += __shfl_down_sync(0xffffffffu, t[c], o);
+        if (lane == 0) sums[warp][c] = t[c];
+    }
+    __syncthreads();
+    if (tid < 3) {
+        double u = 0.0;
+        for (int w = 0; w < 8; ++w) u += sums[w][tid];
+        out[tid] = u;
+    }
+}
+
+template <typename T>
+cudaError_t launch_single_impl(StepParams<T>& p, const uint8_t* mask, const double grad[3], int vel, int prec, cudaStream_t s) {
+    const int n = p.nx * p.ny * p.nz, ctas = std::min((n + PT - 1) / PT, SINGLE_CTAS);
+    const double3 g = make_double3(grad[0], grad[1], grad[2]);
+    p.pchunks = (uint32_t)ctas;
+    p.by_pitch = make_fast_div((uint32_t)p.nx);
+    p.by_ny = make_fast_div((uint32_t)p.ny);
+    if (vel) {
+        if (prec) single_step_kernel<T, true, true><<<ctas, PT, 0, s>>>(p, mask, g);
+        else single_step_kernel<T, true, false><<<ctas, PT, 0, s>>>(p, mask, g);
+    } else {
+        if (prec) single_step_kernel<T, false, true><<<ctas, PT, 0, s>>>(p, mask, g);
+        else single_step_kernel<T, false, false><<<ctas, PT, 0, s>>>(p, mask, g);
+    }
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = pdl_config(dim3(1), dim3(256), 0, s, attr);
+    return cudaLaunchKernelEx(&cfg, single_finish_kernel<T>, (const double*)p.partials, ctas, p.mt);
+}
+
+}  // namespace bt
