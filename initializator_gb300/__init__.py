@@ -297,10 +297,13 @@ class Solver:
         hs.synchronize()
 
     def get_state(self):
-        comps = [np.zeros((self.batch,) + self.shape) for _ in range(3)]
+        if self.batch == 1:
+            out = np.empty((3,) + self.shape)
+            self._check(self._l.bt_get_state(self._h, _dp(out[0]), _dp(out[1]), _dp(out[2])), "get_state")
+            return out
+        comps = [np.empty((self.batch,) + self.shape) for _ in range(3)]
         self._check(self._l.bt_get_state(self._h, _dp(comps[0]), _dp(comps[1]), _dp(comps[2])), "get_state")
-        out = np.stack(comps, axis=1)
-        return out[0] if self.batch == 1 else out
+        return np.stack(comps, axis=1)
 
     def set_schedule(self, pulses=(), grad_wave=None):
         arr = (Pulse * max(1, len(pulses)))()

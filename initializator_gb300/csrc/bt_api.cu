@@ -65,9 +65,10 @@ struct bt_handle {
     // steps run returns once it is converted) up to 2^26 voxels, two above
     int nstage = 2;
     cudaEvent_t stage_ev[3] = {}; // the last copy through each slot
-    // FP32 single fields with three staging slots: bt_set_state copies into
-    // an inbox on a stream of its own (so the copy runs beside steps still
-    // queued) and the handle's stream moves it into the field after them
+    // three dense components that fields cross to and from the host through, up
+    // to 2^26 voxels; bt_set_state of FP32 single fields copies into it on a
+    // stream of its own (so the copy runs beside steps still queued) and the
+    // handle's stream moves it into the field after them
     void* inbox = nullptr;
     bool no_inbox = false;        // no room for it on the device
     cudaStream_t xfer = nullptr;
@@ -1071,16 +1072,56 @@ int put_component(bt_handle* h, void* dst, const double* src, int half, cudaStre
     return BT_OK;
 }
 
+// the inbox, allocated when it is first needed; without room for it (or above
+// 2^26 voxels) fields cross row by row
+bool ensure_inbox(bt_handle* h) {
+    if (h->no_inbox || h->nvox > ((size_t)1 << 26)) return false;
+    if (!h->inbox && cudaMalloc(&h->inbox, 3 * h->nvox * h->esz) != cudaSuccess) {
+        cudaGetLastError();
+        h->inbox = nullptr;
+        h->no_inbox = true;
+    }
+    return h->inbox != nullptr;
+}
+void* inbox_slot(bt_handle* h, int a) { return (char*)h->inbox + (size_t)a * h->nvox * h->esz; }
+
+// host FP64 component -> inbox slot a, as put_component
+int put_inbox(bt_handle* h, int a, const double* src, int half, cudaStream_t s) {
+    if (h->esz == 8) {
+        CK(h, cudaMemcpyAsync(inbox_slot(h, a), src, h->nvox * 8, cudaMemcpyHostToDevice, s));
+    } else {
+        float* f = static_cast<float*>(h->staging) + (size_t)half * h->nvox;
+        CK(h, cudaEventSynchronize(h->stage_ev[half]));
+        convert(f, src, h->nvox);
+        CK(h, cudaMemcpyAsync(inbox_slot(h, a), f, h->nvox * 4, cudaMemcpyHostToDevice, s));
+        CK(h, cudaEventRecord(h->stage_ev[half], s));
+    }
+    return BT_OK;
+}
+
+// device component -> host memory of the handle's type, dense (through inbox
+// slot a where there is one)
+int take_component(bt_handle* h, void* dst, const void* src, int a) {
+    const bt_config& c = h->cfg;
+    if (!ensure_inbox(h)) {
+        CK(h, cudaMemcpy2DAsync(dst, c.nx * h->esz, src, h->pitch * h->esz, c.nx * h->esz, (size_t)c.ny * c.nz,
+                                cudaMemcpyDeviceToHost, h->stream));
+        return BT_OK;
+    }
+    CK(h, h->esz == 8 ? bt::field_out<double>((double*)inbox_slot(h, a), (const double*)src, c.nx, c.ny, c.nz, h->pitch, h->stream)
+                      : bt::field_out<float>((float*)inbox_slot(h, a), (const float*)src, c.nx, c.ny, c.nz, h->pitch, h->stream));
+    CK(h, cudaMemcpyAsync(dst, inbox_slot(h, a), h->nvox * h->esz, cudaMemcpyDeviceToHost, h->stream));
+    return BT_OK;
+}
+
 // device field components -> host FP64 (n of them): for FP32 handles the copy
 // of component i + 1 into one staging half runs while component i is
 // converted out of the other
 int get_components(bt_handle* h, double* const* dst, const void* const* src, int n) {
-    const bt_config& c = h->cfg;
-    const size_t rows = (size_t)c.ny * c.nz;
+    int rc;
     if (h->esz == 8) {
         for (int i = 0; i < n; ++i)
-            CK(h, cudaMemcpy2DAsync(dst[i], c.nx * 8, src[i], h->pitch * 8, c.nx * 8, rows, cudaMemcpyDeviceToHost,
-                                    h->stream));
+            if ((rc = take_component(h, dst[i], src[i], i % 3))) return rc;
         CK(h, cudaStreamSynchronize(h->stream));
         return BT_OK;
     }
@@ -1089,8 +1130,7 @@ int get_components(bt_handle* h, double* const* dst, const void* const* src, int
         if (i < n) {
             // the half was last read by the conversion of component i - 2, done by now
             float* fi = f + (size_t)(i & 1) * h->nvox;
-            CK(h, cudaMemcpy2DAsync(fi, c.nx * 4, src[i], h->pitch * 4, c.nx * 4, rows, cudaMemcpyDeviceToHost,
-                                    h->stream));
+            if ((rc = take_component(h, fi, src[i], i % 3))) return rc;
             CK(h, cudaEventRecord(h->stage_ev[i & 1], h->stream));
         }
         if (i > 0) {
@@ -1113,19 +1153,20 @@ void take_solid_flag(bt_handle* h) {
 
 // The current field's solid voxels looked over on the device (see solid_flag);
 // with src, the dense device arrays become the field on the way.
-int solid_check(bt_handle* h, const void* const* src) {
+int solid_check(bt_handle* h, const void* const* src, int b0, int members) {
     const bt_config& c = h->cfg;
+    void* field = (char*)h->state_base[h->cur] + (size_t)b0 * 3 * h->comp * h->esz;
     cudaError_t e;
     if (c.precision == BT_F64) {
         const double* s[3] = {src ? (const double*)src[0] : nullptr, src ? (const double*)src[1] : nullptr,
                               src ? (const double*)src[2] : nullptr};
-        e = bt::field_in<double>((double*)h->state_base[h->cur], src ? s : nullptr, h->code, c.nx, c.ny, c.nz, h->pitch,
-                                 h->cpitch, (long long)h->comp, h->nb, h->solid_flag, h->stream);
+        e = bt::field_in<double>((double*)field, src ? s : nullptr, h->code, c.nx, c.ny, c.nz, h->pitch, h->cpitch,
+                                 (long long)h->comp, members, h->solid_flag, h->stream);
     } else {
         const float* s[3] = {src ? (const float*)src[0] : nullptr, src ? (const float*)src[1] : nullptr,
                              src ? (const float*)src[2] : nullptr};
-        e = bt::field_in<float>((float*)h->state_base[h->cur], src ? s : nullptr, h->code, c.nx, c.ny, c.nz, h->pitch,
-                                h->cpitch, (long long)h->comp, h->nb, h->solid_flag, h->stream);
+        e = bt::field_in<float>((float*)field, src ? s : nullptr, h->code, c.nx, c.ny, c.nz, h->pitch, h->cpitch,
+                                (long long)h->comp, members, h->solid_flag, h->stream);
     }
     CK(h, e);
     h->launches++;
@@ -1133,6 +1174,7 @@ int solid_check(bt_handle* h, const void* const* src) {
     h->solid_unknown = false;
     return BT_OK;
 }
+int solid_check(bt_handle* h, const void* const* src) { return solid_check(h, src, 0, h->nb); }
 
 }  // namespace
 
@@ -1312,17 +1354,33 @@ int bt_upload_geometry(bt_handle* h, const uint8_t* mask, const double* vx, cons
         const int p3[3] = {h->vxpitch, h->pitch, h->pitch};
         const size_t rows3[3] = {(size_t)c.ny * c.nz, (size_t)(c.ny + 1) * c.nz, (size_t)c.ny * (c.nz + 1)};
         const double* src[3] = {vx, vy, vz};
-        for (int a = 0; a < 3; ++a) {
+        // in one piece, converted and pitched on the device; row by row where
+        // there is no room for that
+        double* tmp = nullptr;
+        if (cudaMalloc(&tmp, sizeof(double) * std::max({w3[0] * rows3[0], w3[1] * rows3[1], w3[2] * rows3[2]})) !=
+            cudaSuccess) {
+            cudaGetLastError();
+            tmp = nullptr;
+        }
+        e = cudaSuccess;
+        for (int a = 0; a < 3 && e == cudaSuccess; ++a) {
             const size_t n = (size_t)w3[a] * rows3[a];
-            if (h->esz == 8) {
-                CK(h, cudaMemcpy2D(h->vel[a], p3[a] * 8, src[a], w3[a] * 8, w3[a] * 8, rows3[a], cudaMemcpyHostToDevice));
+            if (tmp) {
+                e = cudaMemcpyAsync(tmp, src[a], n * 8, cudaMemcpyHostToDevice, h->stream);
+                if (e == cudaSuccess)
+                    e = h->esz == 8 ? bt::rows_in<double>((double*)h->vel[a], tmp, w3[a], p3[a], (long long)rows3[a], h->stream)
+                                    : bt::rows_in<float>((float*)h->vel[a], tmp, w3[a], p3[a], (long long)rows3[a], h->stream);
+            } else if (h->esz == 8) {
+                e = cudaMemcpy2D(h->vel[a], p3[a] * 8, src[a], w3[a] * 8, w3[a] * 8, rows3[a], cudaMemcpyHostToDevice);
             } else {
                 std::vector<float> f(n);
                 convert(f.data(), src[a], n);
-                CK(h, cudaMemcpy2D(h->vel[a], p3[a] * 4, f.data(), w3[a] * 4, w3[a] * 4, rows3[a],
-                                   cudaMemcpyHostToDevice));
+                e = cudaMemcpy2D(h->vel[a], p3[a] * 4, f.data(), w3[a] * 4, w3[a] * 4, rows3[a], cudaMemcpyHostToDevice);
             }
         }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+        cudaFree(tmp);
+        CK(h, e);
     }
     // a field from before the new geometry may hold something where there is
     // solid now
@@ -1349,51 +1407,44 @@ int bt_set_state(bt_handle* h, const double* mx, const double* my, const double*
     if (!h || !mx || !my || !mz) return fail(h, BT_E_ARG, "null field");
     if (!h->geometry) return fail(h, BT_E_STATE, "bt_upload_geometry first");
     const double* src[3] = {mx, my, mz};
-    bool use_inbox = h->esz == 4 && h->nb == 1 && h->nstage == 3 && !h->no_inbox;
-    if (use_inbox && !h->inbox && cudaMalloc(&h->inbox, 3 * h->comp * 4) != cudaSuccess) {
-        // the inbox only overlaps copies with steps: without room for it the
-        // copies go straight into the field
-        cudaGetLastError();
-        h->inbox = nullptr;
-        h->no_inbox = true;
-        use_inbox = false;
-    }
-    if (use_inbox) {
-        // through the inbox: the host-to-device copies run on the transfer
-        // stream beside any steps still queued, then one device copy moves
-        // the field in after them
-        if (!h->xfer) {
-            CK(h, cudaMemset(h->inbox, 0, 3 * h->comp * 4));  // the pitch padding stays zero
+    int rc;
+    if (ensure_inbox(h)) {
+        // FP32 single fields: the host-to-device copies run on the transfer
+        // stream beside any steps still queued; the kernel that moves the field
+        // in (and looks its solid voxels over) comes after them
+        const bool own = h->esz == 4 && h->nb == 1;
+        if (own && !h->xfer) {
             CK(h, cudaStreamCreateWithFlags(&h->xfer, cudaStreamNonBlocking));
             CK(h, cudaEventCreateWithFlags(&h->in_ready, cudaEventDisableTiming));
             CK(h, cudaEventCreateWithFlags(&h->inbox_free, cudaEventDisableTiming));
             CK(h, cudaEventRecord(h->inbox_free, h->stream));
         }
-        CK(h, cudaStreamWaitEvent(h->xfer, h->inbox_free, 0));  // the previous move out of the inbox
-        for (int a = 0; a < 3; ++a) {
-            int rc = put_component(h, (char*)h->inbox + (size_t)a * h->comp * 4, src[a], a, h->xfer);
-            if (rc) return rc;
+        if (own) CK(h, cudaStreamWaitEvent(h->xfer, h->inbox_free, 0));  // the previous move out of the inbox
+        const void* in[3] = {inbox_slot(h, 0), inbox_slot(h, 1), inbox_slot(h, 2)};
+        for (int b = 0; b < h->nb; ++b) {
+            for (int a = 0; a < 3; ++a)
+                if ((rc = put_inbox(h, a, src[a] + (size_t)b * h->nvox, a, own ? h->xfer : h->stream))) return rc;
+            if (own) {
+                CK(h, cudaEventRecord(h->in_ready, h->xfer));
+                CK(h, cudaStreamWaitEvent(h->stream, h->in_ready, 0));
+            }
+            if ((rc = solid_check(h, in, b, 1))) return rc;
         }
-        CK(h, cudaEventRecord(h->in_ready, h->xfer));
-        CK(h, cudaStreamWaitEvent(h->stream, h->in_ready, 0));
-        CK(h, cudaMemcpyAsync(h->state_base[h->cur], h->inbox, 3 * h->comp * 4, cudaMemcpyDeviceToDevice, h->stream));
-        CK(h, cudaEventRecord(h->inbox_free, h->stream));
+        if (own) CK(h, cudaEventRecord(h->inbox_free, h->stream));
     } else {
         for (int b = 0; b < h->nb; ++b)
             for (int a = 0; a < 3; ++a) {
                 void* dst = (char*)h->state[h->cur][a] + (size_t)b * 3 * h->comp * h->esz;
-                int rc = put_component(h, dst, src[a] + (size_t)b * h->nvox, (3 * b + a) % h->nstage, h->stream);
-                if (rc) return rc;
+                if ((rc = put_component(h, dst, src[a] + (size_t)b * h->nvox, (3 * b + a) % h->nstage, h->stream)))
+                    return rc;
             }
+        if ((rc = solid_check(h, nullptr))) return rc;
     }
-    int rcf = solid_check(h, nullptr);
-    if (rcf) return rcf;
     // FP32: the host arrays have been read (converted into the staging
     // slots); the copies and the frame change complete in the handle's
     // stream order. FP64 copies read the caller's arrays directly, so they
     // finish before the call returns.
-    int rc = frame_change(h, h->state[h->cur], +1);
-    if (rc) return rc;
+    if ((rc = frame_change(h, h->state[h->cur], +1))) return rc;
     if (h->esz == 8) CK(h, cudaStreamSynchronize(h->stream));
     return BT_OK;
 }

@@ -290,6 +290,26 @@ __global__ void field_in_kernel(T* field, const T* s0, const T* s1, const T* s2,
     if (bad == 3) atomicOr(flag, 3);
 }
 
+// one component of the field as a dense array
+template <typename T>
+__global__ void field_out_kernel(T* dense, const T* comp, int nx, int pitch, long long rows) {
+    const long long n = rows * nx;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const long long row = q / nx;
+        dense[q] = comp[row * pitch + (q - row * nx)];
+    }
+}
+
+// dense FP64 rows of `width` into pitched rows of the handle's type
+template <typename T>
+__global__ void rows_in_kernel(T* dst, const double* src, int width, int pitch, long long rows) {
+    const long long n = rows * width;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const long long row = q / width;
+        dst[row * pitch + (q - row * width)] = (T)src[q];
+    }
+}
+
 // zero in the solid voxels of a field
 template <typename T>
 __global__ void solid_clear_kernel(T* field, const uint8_t* code, int nx, int ny, int nz, int pitch, int cpitch,
@@ -362,6 +382,21 @@ cudaError_t field_in(T* field, const T* const* src, const uint8_t* code, int nx,
 }
 
 template <typename T>
+cudaError_t field_out(T* dense, const T* comp, int nx, int ny, int nz, int pitch, cudaStream_t s) {
+    const long long rows = (long long)ny * nz, n = rows * nx;
+    const int blocks = (int)std::min<long long>((n + 255) / 256, 152 * 8);
+    field_out_kernel<T><<<blocks, 256, 0, s>>>(dense, comp, nx, pitch, rows);
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t rows_in(T* dst, const double* src, int width, int pitch, long long rows, cudaStream_t s) {
+    const int blocks = (int)std::min<long long>((rows * width + 255) / 256, 152 * 8);
+    rows_in_kernel<T><<<blocks, 256, 0, s>>>(dst, src, width, pitch, rows);
+    return cudaGetLastError();
+}
+
+template <typename T>
 cudaError_t solid_clear(T* field, const uint8_t* code, int nx, int ny, int nz, int pitch, int cpitch, long long comp,
                         int members, cudaStream_t s) {
     const long long n = (long long)(pitch / 4) * ny * nz;
@@ -374,6 +409,10 @@ template cudaError_t field_in<float>(float*, const float* const*, const uint8_t*
                                      int*, cudaStream_t);
 template cudaError_t field_in<double>(double*, const double* const*, const uint8_t*, int, int, int, int, int, long long,
                                       int, int*, cudaStream_t);
+template cudaError_t field_out<float>(float*, const float*, int, int, int, int, cudaStream_t);
+template cudaError_t field_out<double>(double*, const double*, int, int, int, int, cudaStream_t);
+template cudaError_t rows_in<float>(float*, const double*, int, int, long long, cudaStream_t);
+template cudaError_t rows_in<double>(double*, const double*, int, int, long long, cudaStream_t);
 template cudaError_t solid_clear<float>(float*, const uint8_t*, int, int, int, int, int, long long, int, cudaStream_t);
 template cudaError_t solid_clear<double>(double*, const uint8_t*, int, int, int, int, int, long long, int, cudaStream_t);
 
