@@ -182,7 +182,11 @@ __device__ __forceinline__ void far_cells(const Cell& v, int nx, int ny, int nz,
     far[5] = (long long)v.y * pitch + v.x;
 }
 
-template <typename T, int SCHEME, bool VEL, bool PREC, bool PHS>
+// FLD: per-voxel rates and face diffusivities, known when the kernel is built, so
+// that no branch keeps their loads from going out with the others (128 x 112 x 96
+// FP32 with flow and the two-component sums, us a step: 37 with a branch a load,
+// 35 with the next entry's index read ahead, 31 with both)
+template <typename T, int SCHEME, bool VEL, bool PREC, bool PHS, bool FLD>
 __global__ void __launch_bounds__(PT, list_ctas_per_sm(sizeof(T))) pore_step_kernel(const __grid_constant__ StepParams<T> P) {
     constexpr int NS = PHS ? 9 : 3;
     __shared__ double sums[NS][PT];
@@ -252,9 +256,20 @@ __global__ void __launch_bounds__(PT, list_ctas_per_sm(sizeof(T))) pore_step_ker
     Acc2 acc6f[PHS ? 6 : 1];
     double acc6[PHS ? 6 : 1] = {};
 
+    // the next entry is read ahead: everything else of it hangs on its index
+    uint32_t ahead = 0;
+    int code = 0;
+    if (k.first + tid < k.last) {
+        ahead = P.pidx[k.first + tid];
+        code = P.pcode[k.first + tid];
+    }
     for (uint32_t i = k.first + tid; i < k.last; i += PT) {
-        const uint32_t q = P.pidx[i];
-        const int f = P.pcode[i] & 63;
+        const uint32_t q = ahead;
+        const int f = code & 63;
+        if (i + PT < k.last) {
+            ahead = P.pidx[i + PT];
+            code = P.pcode[i + PT];
+        }
         const Cell v = cell_of(q, P.by_pitch, P.by_ny, pitch, ny);
         bool open[6] = {v.x > 0, v.x < nx - 1, v.y > 0, v.y < ny - 1, v.z > 0, v.z < nz - 1};
         T p0[3], nb[3][6];
@@ -270,8 +285,8 @@ __global__ void __launch_bounds__(PT, list_ctas_per_sm(sizeof(T))) pore_step_ker
             vf[4] = P.vz[q];
             vf[5] = P.vz[q + plane];
         }
-        T dtt1 = P.fdtt ? P.fdtt[q] : P.dtt1[f], dtt2 = P.fdtt ? P.fdtt[P.fstride + q] : P.dtt2[f];
-        if (P.pal) {
+        T dtt1 = FLD || P.fdtt ? P.fdtt[q] : P.dtt1[f], dtt2 = FLD || P.fdtt ? P.fdtt[P.fstride + q] : P.dtt2[f];
+        if (!FLD && P.pal) {
             // FP32 per-voxel rates through the rate palette
             const int id = P.pal_idx[((long long)v.z * ny + v.y) * P.cpitch + v.x];
             dtt1 = (T)P.pal[2 * id];
@@ -279,7 +294,7 @@ __global__ void __launch_bounds__(PT, list_ctas_per_sm(sizeof(T))) pore_step_ker
         }
         T df[6];
 #pragma unroll
-        for (int a = 0; a < 6; ++a) df[a] = P.fw ? P.fw[a * P.fstride + q] : (f & (1 << a)) ? P.dps : P.dpp;
+        for (int a = 0; a < 6; ++a) df[a] = FLD || P.fw ? P.fw[a * P.fstride + q] : (f & (1 << a)) ? P.dps : P.dpp;
         T w1 = 0, w2 = 0;
         if constexpr (PHS) {
             w1 = P.phw[q];
@@ -416,9 +431,20 @@ __global__ void __launch_bounds__(PT, list_ctas_per_sm(sizeof(T))) pore_mac_kern
     Acc2 acc6f[PHS ? 6 : 1];
     double acc6[PHS ? 6 : 1] = {};
 
+    // the next entry is read ahead: everything else of it hangs on its index
+    uint32_t ahead = 0;
+    int code = 0;
+    if (k.first + tid < k.last) {
+        ahead = P.pidx[k.first + tid];
+        code = P.pcode[k.first + tid];
+    }
     for (uint32_t i = k.first + tid; i < k.last; i += PT) {
-        const uint32_t q = P.pidx[i];
-        const int f = P.pcode[i] & 63;
+        const uint32_t q = ahead;
+        const int f = code & 63;
+        if (i + PT < k.last) {
+            ahead = P.pidx[i + PT];
+            code = P.pcode[i + PT];
+        }
         const Cell v = cell_of(q, P.by_pitch, P.by_ny, pitch, ny);
         bool open[6] = {v.x > 0, v.x < nx - 1, v.y > 0, v.y < ny - 1, v.z > 0, v.z < nz - 1};
         T p0[3], nb[3][6];
@@ -567,10 +593,13 @@ cudaError_t launch_list_kernel(K kernel, const StepParams<T>& p, size_t smem, cu
 
 // the KSPACE kernel's phase tables need more than the 48 KB a kernel gets by
 // default on grids whose edges add up to thousands
-template <typename T, int SCHEME, bool VEL, bool PREC, bool PHS>
+template <typename T, int SCHEME, bool VEL, bool PREC, bool PHS, bool FLD = false>
 cudaError_t launch_pore_step(const StepParams<T>& p, cudaStream_t s) {
+    // (FP64 is bound by its arithmetic: one form)
+    if constexpr (sizeof(T) == 4 && SCHEME == SCHEME_REF && !FLD)
+        if (p.fdtt && p.fw && !p.pal) return launch_pore_step<T, SCHEME, VEL, PREC, PHS, true>(p, s);
     const size_t smem = SCHEME == SCHEME_KSPACE ? 2 * sizeof(T) * ((size_t)p.nx + p.ny + p.nz) : 0;
-    auto kernel = pore_step_kernel<T, SCHEME, VEL, PREC, PHS>;
+    auto kernel = pore_step_kernel<T, SCHEME, VEL, PREC, PHS, FLD>;
     if (smem > 40 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
