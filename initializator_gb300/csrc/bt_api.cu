@@ -128,6 +128,7 @@ struct bt_handle {
     int phase_axes = bt::PH_ALL;  // KSPACE: axes with a wave vector somewhere in the schedule
     // the pore list (bt_list.cuh) of the generic kernels, and its chunks
     bool use_list = false;
+    bool no_list = false;         // no room for it
     uint32_t* pidx = nullptr;
     uint8_t* pcode = nullptr;
     int* pbox = nullptr;
@@ -451,15 +452,15 @@ void free_pore_list(bt_handle* h) {
     h->pidx = nullptr;
     h->pcode = nullptr;
     h->pbox = nullptr;
-    h->use_list = false;
+    h->use_list = h->no_list = false;
 }
 
 int build_pore_list(bt_handle* h) {
     const bt_config& c = h->cfg;
     const uint32_t nseg = bt::list_segments(c.nx, c.ny, c.nz);
     uint32_t* offs = nullptr;
-    CK(h, cudaMalloc(&offs, sizeof(uint32_t) * ((size_t)nseg + 1)));
-    cudaError_t e = bt::list_offsets(h->code, c.nx, c.ny, c.nz, h->cpitch, false, offs, h->stream);
+    cudaError_t e = cudaMalloc(&offs, sizeof(uint32_t) * ((size_t)nseg + 1));
+    if (e == cudaSuccess) e = bt::list_offsets(h->code, c.nx, c.ny, c.nz, h->cpitch, false, offs, h->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h->npore, offs + nseg, 4, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     const size_t n = std::max<size_t>(1, h->npore);
@@ -477,6 +478,13 @@ int build_pore_list(bt_handle* h) {
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     cudaFree(offs);
+    if (e == cudaErrorMemoryAllocation) {
+        // the dense kernels need no list
+        cudaGetLastError();
+        free_pore_list(h);
+        h->no_list = true;
+        return BT_OK;
+    }
     CK(h, e);
     int rc = grow_partials(h, 6 * (size_t)h->pchunks * h->nb);
     if (rc) return rc;
@@ -543,8 +551,8 @@ int build_quad_list(bt_handle* h) {
     if (c.scheme == BT_SCHEME_KSPACE && 8 * ((size_t)c.nx + c.ny + c.nz + 4) > 160 * 1024) return BT_OK;
     const uint32_t nseg = bt::list_segments(c.nx, c.ny, c.nz);
     uint32_t* offs = nullptr;
-    CK(h, cudaMalloc(&offs, sizeof(uint32_t) * ((size_t)nseg + 1)));
-    cudaError_t e = bt::list_offsets(h->code, c.nx, c.ny, c.nz, h->cpitch, true, offs, h->stream);
+    cudaError_t e = cudaMalloc(&offs, sizeof(uint32_t) * ((size_t)nseg + 1));
+    if (e == cudaSuccess) e = bt::list_offsets(h->code, c.nx, c.ny, c.nz, h->cpitch, true, offs, h->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h->nquad, offs + nseg, 4, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess && ring_is_faster(h)) {
@@ -559,6 +567,12 @@ int build_quad_list(bt_handle* h) {
     if (e == cudaSuccess && c.velocity == 1) e = cudaMalloc(&h->qvel, sizeof(float) * 12 * n);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     cudaFree(offs);
+    if (e == cudaErrorMemoryAllocation) {
+        // the ring needs no list
+        cudaGetLastError();
+        free_quads(h);
+        return BT_OK;
+    }
     CK(h, e);
     h->quad_ok = h->use_quad = true;
     int rc = default_quad_chunks(h);
@@ -570,10 +584,18 @@ int build_quad_list(bt_handle* h) {
     return BT_OK;
 }
 
+int ensure_ring(bt_handle* h);
+
 // the uploaded rate palette's indices in list order
 int quad_rates(bt_handle* h) {
     if (!h->quad_ok) return BT_OK;
-    if (!h->qpal) CK(h, cudaMalloc(&h->qpal, 4 * std::max<size_t>(1, h->nquad)));
+    if (!h->qpal && cudaMalloc(&h->qpal, 4 * std::max<size_t>(1, h->nquad)) != cudaSuccess) {
+        cudaGetLastError();
+        free_quads(h);  // the ring reads the indices where they are
+        const int rc = ensure_ring(h);
+        refresh_params(h);
+        return rc;
+    }
     CK(h, bt::quad_palette(h->qhead, h->nquad, h->pal_idx, h->pitch, h->cpitch, h->qpal, h->stream));
     return BT_OK;
 }
@@ -1526,7 +1548,7 @@ int run_begin(bt_handle* h, long long nsteps) {
     take_solid_flag(h);
     h->touched = true;
     // the generic kernels' list, built when they are first needed
-    if (!h->use_list && list_possible(h) && generic_steps(h) && (rc = build_pore_list(h))) return rc;
+    if (!h->use_list && !h->no_list && list_possible(h) && generic_steps(h) && (rc = build_pore_list(h))) return rc;
     h->ctl_h->step = h->step;
     h->ctl_h->mt_base = h->step;
     h->ctl_h->ticket = 0;
