@@ -486,7 +486,7 @@ def hbm_peak():
 
 def profiled_traffic():
     """DRAM bytes per launch of the step kernel from the committed ncu summary."""
-    p = os.path.join(ROOT, "profiles", "step_kernel_kspace_256.md")
+    p = os.path.join(ROOT, "profiles", "quad_step_kernel_256.md")
     try:
         with open(p) as f:
             m = re.search(r"dram_bytes_per_launch:\s*([0-9.eE+]+)", f.read())

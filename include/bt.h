@@ -110,7 +110,7 @@ typedef struct bt_config {
  * rotation by param about axis; flags 3 and 4 as the reference. The
  * KSPACE scheme accepts flag 2 only (gradients come from the waveform).
  * Several pulses of one step apply in the order given. On FP32 handles a
- * step whose pulses are all flag 2 stays on the TMA fast path (their product
+ * step whose pulses are all flag 2 stays on the FP32 fast path (their product
  * rotation, formed in FP64, applied in FP32); other pulse steps, and pulse
  * steps of handles with a rate palette, run on the generic kernel. */
 typedef struct bt_pulse {
@@ -192,7 +192,7 @@ int bt_run_async(bt_handle* h, long long nsteps);
  * configuration's d_pore (solid voxels
  * at most 1e-20 m^2/s) and whose pore voxels' FP32 rate pairs take at most 256
  * values keep them as a rate palette (an 8-bit index per voxel, the code
- * table's face weights) and stay on the TMA fast path; other rates run on
+ * table's face weights) and stay on the FP32 fast path; other rates run on
  * the generic kernel, which reads the eight per-voxel fields. */
 int bt_upload_rates(bt_handle* h, const double* t1, const double* t2, const double* diff);
 /* Per-voxel rates given as a palette (no reference counterpart; the same
@@ -221,7 +221,7 @@ int bt_read_mt_phases(bt_handle* h, double* out, long long nsteps);
  * geometry and schedule) by nsteps each, asynchronously. Launches are
  * interleaved round robin, one captured graph of steps per handle per round,
  * so small grids on the handles' separate streams run side by side on the
- * GPU; the handles' FP32 fast paths get z-chunks for sharing the GPU (see
+ * GPU; the handles' FP32 fast paths get chunks for sharing the GPU (see
  * bt_set_tma_split). Read each handle's M(t) with bt_read_mt. No reference
  * counterpart: the reference runs one sample per process (main.cpp:34-36). */
 int bt_run_many(bt_handle* const* hs, int n, long long nsteps);
@@ -233,7 +233,8 @@ void* bt_stream(bt_handle* h);
 /* M(t) sums of the current field (OutputX/Y/Z, cpp:3301-3461). */
 int bt_measure(bt_handle* h, double* sums3);
 
-/* Pick the z-chunking of the FP32 fast path by timing trial_steps steps for
+/* Pick the chunking of the FP32 fast path (CTAs over the list of voxel groups,
+ * or z-chunks of the plane ring that large dense fields take) by timing trial_steps steps for
  * each candidate (no reference counterpart: the reference launches one
  * thread per voxel, cu:1475-1476): for one to eight waves of CTAs (and for a
  * batch the first wave counts that give every tile column a chunk), the chunk
@@ -242,21 +243,24 @@ int bt_measure(bt_handle* h, double* sums3);
  * the chosen number of chunks per field (as for bt_set_tma_chunks). */
 int bt_autotune(bt_handle* h, int trial_steps, int* best_chunks);
 
-/* The FP32 fast path's z-chunking: zsplit chunks per column (<= 0: the
- * default for a handle running alone, about four waves of CTAs). A no-op for
+/* The FP32 fast path's chunking: zsplit chunks per column (<= 0: the
+ * default for a handle running alone: one wave of CTAs over the list, two of the
+ * plane ring). A no-op for
  * handles without the fast path. bt_run_many sets the chunking of its handles
  * for sharing the GPU (about two waves over all of them together); this call
  * (or bt_autotune) sets it back for running alone. */
 int bt_set_tma_split(bt_handle* h, int zsplit);
-/* The FP32 fast path's z-chunking as a number of chunks per field in total:
- * the tile columns get chunks/tiles or one more (so any count of CTAs, e.g.
+/* The FP32 fast path's chunking as a number of chunks per field in total: even
+ * shares of the list (one to one a 128 groups); in the plane ring the tile
+ * columns get chunks/tiles or one more (so any count of CTAs, e.g.
  * exactly two waves, can be launched), clamped to at least one chunk per
  * column and chunks of 1..1024 planes; <= 0: the default. A no-op for handles
  * without the fast path. */
 int bt_set_tma_chunks(bt_handle* h, int chunks);
 
-/* Failure injection for tests (no reference counterpart): the FP32 fast
- * path's plane-ring waits (mbarrier polls for a plane's TMA copy, and the
+/* Failure injection for tests (no reference counterpart): the handle's FP32
+ * steps take the fast path's plane ring (the list of voxel groups has no waits),
+ * and the ring's waits (mbarrier polls for a plane's TMA copy, and the
  * producer's wait for a free ring slot) give up after `polls` polls, 0 = at
  * once, so that a test sees the bounded-wait path run: every CTA that gives
  * up raises its failure flag, waits (with the full bound) for its own copies

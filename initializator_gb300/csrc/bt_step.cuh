@@ -16,6 +16,10 @@
 // In double precision (built with -fmad=false) every expression keeps the
 // reference's operation order, so the field matches it bit for bit.
 //
+// The arithmetic (voxel_step) is shared with the kernels over the pore list
+// (bt_step_pore.cuh), which take every step of grids their 31-bit index reaches
+// and memory has room for; step_kernel below is the dense form for the others.
+//
 // Layout: a CTA owns TX x TY columns and marches through its z-chunk. The
 // voxel's own column rolls through registers (below / current / above); the
 // current plane plus a one-voxel x/y halo sits in shared memory. The sums

@@ -1,4 +1,6 @@
-// FP32 fast path of the fused step (K1, TMA form) for sm_103a.
+// FP32 fast path of the fused step (K1, TMA form) for sm_103a: of fields beyond L2
+// whose groups of four voxels nearly all hold a pore voxel (ring_is_faster in
+// bt_api.cu); the others take the list of those groups (bt_step_quad.cuh).
 //
 // Same update and M(t) as step_kernel (bt_step.cuh), for steps without pulses
 // and steps whose pulses are all fixed-angle (the RF instances apply the
