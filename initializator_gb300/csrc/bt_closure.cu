@@ -690,6 +690,7 @@ int bt_conv3d(const bt_conv3d_args* a, void* stream) {
     if ((a->mode == 0 || a->mode == 1) && !a->bias) return BT_E_ARG;
     if (a->mode == 2 && !a->pre) return BT_E_ARG;
     if (((uintptr_t)a->x | (uintptr_t)a->wpack) & 15u) return BT_E_CUDA;  // 16-byte copies
+    if ((a->mode == 0 || a->mode == 2) && ((uintptr_t)a->out & 15u)) return BT_E_CUDA;  // 16-byte stores
     const int xp = a->nx + 2, yp = a->ny + 2, zp = a->nz + 2;
     ConvParams P{};
     P.xp = xp;
