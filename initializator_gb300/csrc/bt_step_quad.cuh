@@ -92,6 +92,20 @@ __global__ void __launch_bounds__(PT, QUAD_CTAS_PER_SM) quad_step_kernel(const _
     const StepInfo* si = P.steps + (step < P.nsched ? step : P.nsched) * nbt + k.b;
     const float* in[3] = {P.in[0] + k.b * P.bstride, P.in[1] + k.b * P.bstride, P.in[2] + k.b * P.bstride};
     float* out[3] = {P.out[0] + k.b * P.bstride, P.out[1] + k.b * P.bstride, P.out[2] + k.b * P.bstride};
+    // With flow the six pointers do not fit the 128 registers beside the
+    // velocities: their bases come from constant memory (no spills; 192 x 192 x 128
+    // random field, batch of eight, 150 -> 148 us a step, 512 x 384 x 256 159 -> 155).
+    // Without flow the pointers stay in registers (twelve samples of 48 to 192 voxels a
+    // side 145 against 158 us).
+    const unsigned long long member = k.b * (unsigned long long)P.bstride;
+    auto in_at = [&](int c, uint32_t q) -> const float* {
+        if constexpr (VEL) return P.in[c] + (member + 4ull * q);
+        else return in[c] + 4ull * q;
+    };
+    auto out_at = [&](int c, uint32_t q) -> float* {
+        if constexpr (VEL) return P.out[c] + (member + 4ull * q);
+        else return out[c] + 4ull * q;
+    };
     if constexpr (RF) {
         if (tid < 9) s_rot[tid] = si->rotf[tid];
     }
@@ -126,8 +140,8 @@ __global__ void __launch_bounds__(PT, QUAD_CTAS_PER_SM) quad_step_kernel(const _
 
     // rows with an open face towards a quad
     auto open_any = [](uint32_t bits, int f) { return ((bits >> 6) & ~(bits >> f) & 0x00204081u) != 0u; };
-    auto load4 = [](float (&d)[4], const float* p, uint32_t q) {
-        const float4 v = load_row(p + 4ull * q);
+    auto load4 = [](float (&d)[4], const float* p) {
+        const float4 v = load_row(p);
         d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
     };
 
@@ -181,28 +195,28 @@ __global__ void __launch_bounds__(PT, QUAD_CTAS_PER_SM) quad_step_kernel(const _
         float hl[3] = {0.f, 0.f, 0.f}, hr[3] = {0.f, 0.f, 0.f};
         if (load_l && (bits & 0x41u) == 0x40u) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) hl[c] = in[c][4ull * quad - 1];
+            for (int c = 0; c < 3; ++c) hl[c] = in_at(c, quad)[-1];
         }
         if (load_r && (bits & (0x42u << 21)) == (0x40u << 21)) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) hr[c] = in[c][4ull * quad + 4];
+            for (int c = 0; c < 3; ++c) hr[c] = in_at(c, quad)[4];
         }
         float cur[3][4], xl[3], xr[3], ym[3][4], yp[3][4], zm[3][4], zp[3][4];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            load4(cur[c], in[c], quad);
-            load4(zp[c], in[c], ozp);
-            load4(ym[c], in[c], oym);
-            load4(yp[c], in[c], oyp);
-            load4(zm[c], in[c], ozm);
+            load4(cur[c], in_at(c, quad));
+            load4(zp[c], in_at(c, ozp));
+            load4(ym[c], in_at(c, oym));
+            load4(yp[c], in_at(c, oyp));
+            load4(zm[c], in_at(c, ozm));
         }
         float u[3][4] = {};
         if constexpr (VEL) {
             // (of entries beyond the block: any velocity, they are zeros throughout)
             const float* qv = P.qvel + 4ull * min(i, P.nquad - 1u);
-            load4(u[0], qv, 0u);
-            load4(u[1], qv, P.nquad);
-            load4(u[2], qv, 2u * P.nquad);
+            load4(u[0], qv);
+            load4(u[1], qv + 4ull * P.nquad);
+            load4(u[2], qv + 8ull * P.nquad);
         }
         uint32_t pal4 = 0;
         if constexpr (PAL) {
@@ -250,8 +264,8 @@ __global__ void __launch_bounds__(PT, QUAD_CTAS_PER_SM) quad_step_kernel(const _
             if (x == 0) {
                 if (kx == BC_COPY) ghost(xl[0], xl[1], xl[2], cur[0][0], cur[1][0], cur[2][0], 0, false);
                 if (kx == BC_PERIODIC) {
-                    const size_t o = 4ull * rowq + (nx - 1);
-                    wrap(xl[0], xl[1], xl[2], in[0][o], in[1][o], in[2][o], 0, false);
+                    const int o = nx - 1;
+                    wrap(xl[0], xl[1], xl[2], in_at(0, rowq)[o], in_at(1, rowq)[o], in_at(2, rowq)[o], 0, false);
                 }
             }
 #pragma unroll
@@ -260,8 +274,7 @@ __global__ void __launch_bounds__(PT, QUAD_CTAS_PER_SM) quad_step_kernel(const _
                     float g[3] = {0.f, 0.f, 0.f};
                     if (kx == BC_COPY) ghost(g[0], g[1], g[2], cur[0][j], cur[1][j], cur[2][j], 0, true);
                     if (kx == BC_PERIODIC) {
-                        const size_t o = 4ull * rowq;
-                        wrap(g[0], g[1], g[2], in[0][o], in[1][o], in[2][o], 0, true);
+                        wrap(g[0], g[1], g[2], *in_at(0, rowq), *in_at(1, rowq), *in_at(2, rowq), 0, true);
                     }
 #pragma unroll
                     for (int c = 0; c < 3; ++c) (j < 3 ? nxt[c][j] : xr[c]) = g[c];
@@ -269,7 +282,7 @@ __global__ void __launch_bounds__(PT, QUAD_CTAS_PER_SM) quad_step_kernel(const _
             auto row_ghosts = [&](float (&g)[3][4], int kind, int a, bool upper, uint32_t far) {
                 if (kind == BC_PERIODIC) {
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) load4(g[c], in[c], far);
+                    for (int c = 0; c < 3; ++c) load4(g[c], in_at(c, far));
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -448,14 +461,14 @@ __global__ void __launch_bounds__(PT, QUAD_CTAS_PER_SM) quad_step_kernel(const _
         if (live) {
 #pragma unroll
             for (int c = 0; c < 3; ++c)
-                *reinterpret_cast<float4*>(out[c] + 4ull * quad) = make_float4(o[c][0], o[c][1], o[c][2], o[c][3]);
+                *reinterpret_cast<float4*>(out_at(c, quad)) = make_float4(o[c][0], o[c][1], o[c][2], o[c][3]);
             if (bits & QUAD_ALONE) {
                 // the other quad of this 32-byte sector holds no pore voxel: its
                 // zeros complete the sector, which then goes to HBM without
                 // being read for the rest of it
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
-                    *reinterpret_cast<float4*>(out[c] + 4ull * (quad ^ 1u)) = make_float4(0.f, 0.f, 0.f, 0.f);
+                    *reinterpret_cast<float4*>(out_at(c, quad ^ 1u)) = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
         at = at2;
